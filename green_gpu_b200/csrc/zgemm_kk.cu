@@ -1,0 +1,13 @@
+// FP64 complex GEMM kernels for operands whose contiguous direction is k in A and k in B.
+#include <atomic>
+
+#include "zgemm_kernel.cuh"
+
+namespace gg {
+
+void zgemm_launch_kk(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st) {
+  if (g3) zlaunch_shape<true, true, true>(shape, d, g, teams, st);
+  else zlaunch_shape<true, true, false>(shape, d, g, teams, st);
+}
+
+}  // namespace gg

@@ -1,0 +1,12 @@
+// FP64 complex GEMM kernels for operands whose contiguous direction is m in A and n in B.
+#include <atomic>
+
+#include "zgemm_kernel.cuh"
+
+namespace gg {
+
+void zgemm_launch_nn(int shape, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st) {
+  zlaunch_shape<false, false, false>(shape, d, g, teams, st);
+}
+
+}  // namespace gg
