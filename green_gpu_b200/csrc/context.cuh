@@ -99,7 +99,7 @@ struct gg_context {
 
   // work buffers
   gg::DevBuf<double2> G_in, Sigma_out, Gf, Gtmp, Vbuf, G1buf, scratchA, scratchB, P0buf, Pw, Afac, Wt, Wrot,
-      gemm_work, hf_D, hf_F, hf_c, hf_J;
+      gemm_work, hf_D, hf_F, hf_c, hf_J, lu_inv;
   gg::DevBuf<int> info, piv, idx_i;
   // split precision: exponents of the P0 main contraction's operand rows / columns, recorded
   // by the operand builds' epilogues

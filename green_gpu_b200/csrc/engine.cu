@@ -181,7 +181,7 @@ Plan plan_gw(gg_context* c, int slices) {
   const size_t nn = (size_t)s.nao * s.nao, NN = (size_t)s.NQ * s.NQ, Nnn = (size_t)s.NQ * nn;
   const int T2 = s.nts / 2;
   const size_t held = c->Gf.n + c->Gtmp.n + c->Vbuf.n + c->G1buf.n + c->scratchA.n + c->scratchB.n + c->P0buf.n +
-                      c->Pw.n + c->Afac.n + c->Wt.n + c->Wrot.n + c->gemm_work.n;
+                      c->Pw.n + c->Afac.n + c->Wt.n + c->Wrot.n + c->gemm_work.n + c->lu_inv.n;
   const size_t budget = (size_t)(0.85 * (double)(free_bytes() + held * z));
   Plan p;
   p.dyson_batch = 4 * 148;
@@ -195,7 +195,7 @@ Plan plan_gw(gg_context* c, int slices) {
     b += 2 * std::max(p0s, sgs);
     b += (size_t)q.qc * T2 * NN;                       // P0
     b += (size_t)q.qc * s.nw_b * NN;                   // Pw
-    b += (size_t)std::min<long>(q.dyson_batch, (long)q.qc * s.nw_b) * NN;  // Dyson workspace
+    b += (size_t)std::min<long>(q.dyson_batch, (long)q.qc * s.nw_b) * (NN + 32 * (size_t)s.NQ);  // Dyson workspace
     b += (size_t)q.qc * s.nts * NN;                    // Wt
     b += (size_t)s.nts * NN;                           // Wrot
     b += (size_t)1 << 22;                              // split-K partials
@@ -374,6 +374,8 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
   double2* gw_work = c->gemm_work.ensure((size_t)1 << 22);
   int* info = c->info.ensure((size_t)pl.qc * nw);
   int* piv = solver == GG_SOLVER_LU ? c->piv.ensure((size_t)dys * N) : nullptr;
+  const int lub = dyson_lu_block(N);
+  double2* lu_inv = solver == GG_SOLVER_LU ? c->lu_inv.ensure((size_t)dys * ceil_div(N, lub) * lub * lub) : nullptr;
   std::vector<int> info_h((size_t)pl.qc * nw);
   SplitGemm* split = nullptr;
   if (precision == GG_PREC_SPLIT) split = split_engine(c);
@@ -591,12 +593,11 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
         GG_CUDA(cudaMemcpyAsync((double2*)c->cap_Pw + (long)myq[q0 + qi] * nw * NN, Pw + (long)qi * nw * NN,
                                 (size_t)nw * NN * sizeof(double2), cudaMemcpyDeviceToHost, st));
     }
-    // ---------------- Dyson, FP64, one CTA per (q, W) system
+    // ---------------- Dyson, FP64, all (q, W) systems of a batch together
     h = tm.begin(4);
     for (int s0 = 0; s0 < qn * nw; s0 += dys) {
       const int sn = std::min(dys, qn * nw - s0);
-      launch_dyson(Pw + (long)s0 * NN, Af, info + s0, sn, N, solver, piv, st);
-      ++c->launches;
+      c->launches += launch_dyson(Pw + (long)s0 * NN, Af, lu_inv, info + s0, sn, N, solver, piv, st);
     }
     tm.end(h);
     if (cap) {

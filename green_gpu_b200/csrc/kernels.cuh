@@ -47,8 +47,10 @@ void launch_fill_zero(double2* X, long n, cudaStream_t st);
 // Batched Dyson solve for `nsys` systems of size N x N stored contiguously in P (in place):
 // P <- Hermitian-symmetrise(P); A = I - P; Cholesky: P <- (A^{-1} P)^H, LU: P <- sym(A^{-1} P).
 // `A` is a workspace of the same size, `info` receives per-system status (0 ok; Cholesky:
-// index+1 of the first non-positive pivot; LU: index+1 of the first zero pivot).
-void launch_dyson(double2* P, double2* A, int* info, int nsys, int N, int solver, int* piv_ws, cudaStream_t st);
+// index+1 of the first non-positive pivot; LU: index+1 of the first zero pivot).  LU only: li
+// [nsys][ceil(N / b) b][b] with b = dyson_lu_block(N), piv [nsys][N].  Returns the launches.
+int dyson_lu_block(int N);
+int launch_dyson(double2* P, double2* A, double2* li, int* info, int nsys, int N, int solver, int* piv, cudaStream_t st);
 
 // Hermitian symmetrisation only (cuda_common.cu:249-281), nsys matrices in place.
 void launch_hermitian_symmetrize(double2* P, int nsys, int N, cudaStream_t st);

@@ -71,7 +71,7 @@ ZChoice choose(const ZgemmDesc& d, long batch, long groups, int sms) {
   for (int i = 0; i < count; ++i) {
     const ZShape& s = table[i];
     const int tm = ceil_div(d.M, s.bm), tn = ceil_div(d.N, s.bn);
-    if (d.inplace && tn > 1) continue;
+    if ((d.inplace == 1 && tn > 1) || (d.inplace == 2 && tm > 1)) continue;
     const double tiles = (double)tm * tn * batch;
     const int t88 = s.mt * s.nt;
     const double mma = t88 * prods * 16.0, busy = (0.89 - 0.8 / t88) * (d.gauss ? 0.8 : 1.0);
@@ -93,7 +93,7 @@ ZChoice choose(const ZgemmDesc& d, long batch, long groups, int sms) {
       }
     }
   }
-  if (!have) throw Error(GG_ERR_INTERNAL, "zgemm: no tile shape for an in-place product of this width");
+  if (!have) throw Error(GG_ERR_INTERNAL, "zgemm: no tile shape for an in-place product of this size");
   return best;
 }
 

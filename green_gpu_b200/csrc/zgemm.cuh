@@ -48,8 +48,9 @@ struct ZgemmDesc {
   // 1e-16 relative, but not componentwise).  Used only inside the split-precision build, whose
   // error budget is six orders larger; the FP64 path keeps the four-product form.
   int gauss = 0;
-  // 1: C overlays A (same rows, in the same places): the whole width N is one tile, read before
-  // it is written, and the reduction is not split
+  // C overlays an operand: 1 A (the same rows in the same places, the whole width N is one tile), 2 B
+  // (the same columns, the whole height M is one tile); the operand's tile is read before C's is
+  // written and the reduction is not split
   int inplace = 0;
   int splits = 1;            // split-K factor (deterministic: partials + ordered reduction)
   double2* work = nullptr;   // [splits][batch][M][N] when splits > 1
