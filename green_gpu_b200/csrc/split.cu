@@ -56,6 +56,7 @@ struct SplitGemm {
   };
   std::map<std::array<long, 8>, Choice> tuned;
   std::string report;
+  int b_plane = 0;  // height of the B planes that the last GEMM left in b8
 };
 
 namespace {
@@ -920,6 +921,7 @@ void launch_slices_s(const OpView& va, const OpView& vb, int rows_a_pad, int nco
   slice_kernel<false, S><<<(unsigned)((long)nkb * ((va.R + 31) / 32) * batch_a), 256, 0, st>>>(va, rows_a_pad, nkb, ea,
                                                                                              a8, batch_a);
   GG_CHECK_LAUNCH();
+  if (!b8) return;
   slice_kernel<true, S><<<(unsigned)((long)nkb * ((vb.R + 31) / 32) * batch_b), 256, 0, st>>>(vb, ncol_pad, nkb, eb, b8,
                                                                                           batch_b);
   GG_CHECK_LAUNCH();
@@ -1148,9 +1150,10 @@ int run_planes(SplitGemm* e, const ZgemmDesc& d, int S, const Geometry& g, const
   return launches;
 }
 
-// exponents and slices of both operands into the engine's planes, then the GEMM
+// exponents and slices of both operands into the engine's planes, then the GEMM; keep_b: B's are those
+// that the engine's last GEMM left
 int sliced_gemm(SplitGemm* e, const ZgemmDesc& d, int S, cudaStream_t st, const SplitRowMax* mx = nullptr,
-                const int* ea_given = nullptr, const int* eb_given = nullptr) {
+                const int* ea_given = nullptr, const int* eb_given = nullptr, bool keep_b = false) {
   if (d.M <= 0 || d.N <= 0) return 0;
   Geometry g = geometry(d, S);
   // an operand with zero batch strides is the same matrix for every batch: slice it once
@@ -1181,6 +1184,16 @@ int sliced_gemm(SplitGemm* e, const ZgemmDesc& d, int S, cudaStream_t st, const 
       }
     }
   }
+  // planes of a kept B keep the height they were laid out with (the tuner's are taller); a call that is
+  // tuned lays out its own
+  if (tune || eb_given) keep_b = false;
+  if (keep_b && e->b_plane >= g.rows_b_pad) {
+    g.rows_b_plane = e->b_plane;
+    g.ncol_pad = g.rows_b_plane / 2;
+  } else {
+    keep_b = false;
+  }
+  e->b_plane = g.rows_b_plane;
   int8_t* a8 = e->a8.ensure((size_t)batch_a * S * g.rows_a_pad * g.kp);
   int8_t* b8 = e->b8.ensure((size_t)batch_b * S * g.rows_b_plane * g.kp);
   int* ea = e->ea.ensure((size_t)batch_a * g.rows_a_pad);
@@ -1207,11 +1220,12 @@ int sliced_gemm(SplitGemm* e, const ZgemmDesc& d, int S, cudaStream_t st, const 
   }
   if (eb_given) {
     eb = const_cast<int*>(eb_given);
-  } else {
+  } else if (!keep_b) {
     exponents(vb, d.N, eb, batch_b);
     ++launches;
   }
-  launch_slices(S, va, vb, g.rows_a_pad, g.ncol_pad, g.nkb, ea, eb, a8, b8, batch_a, batch_b, st);
+  if (keep_b) --launches;
+  launch_slices(S, va, vb, g.rows_a_pad, g.ncol_pad, g.nkb, ea, eb, a8, keep_b ? nullptr : b8, batch_a, batch_b, st);
   if (!tune) return launches + run_planes(e, d, S, g, a8, b8, ea, eb, a_shared, b_shared, st, mx, force_splits);
   // time every (width, split-K) candidate on the sliced planes; the rule's split-K factor, one
   // and twice the rule's bracket the split-K choice
@@ -1285,7 +1299,9 @@ SplitPlanes split_planes_for(const ZgemmDesc& d, int S) {
   return p;
 }
 
-int split_zgemm(SplitGemm* e, const ZgemmDesc& d, int S, cudaStream_t st) { return sliced_gemm(e, d, S, st); }
+int split_zgemm(SplitGemm* e, const ZgemmDesc& d, int S, cudaStream_t st, bool keep_b) {
+  return sliced_gemm(e, d, S, st, nullptr, nullptr, nullptr, keep_b);
+}
 
 int split_zgemm_rowmax(SplitGemm* e, const ZgemmDesc& d, int S, const SplitRowMax& mx, cudaStream_t st) {
   if (!mx.on || !mx.ex || mx.div_m < 1 || mx.div_n < 1)

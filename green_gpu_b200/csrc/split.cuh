@@ -31,8 +31,10 @@ SplitPlanes split_planes_for(const ZgemmDesc& d, int S);
 struct SplitGemm;
 // Per-context engine (workspace for slices); throws if the path is unavailable.
 SplitGemm* split_engine(gg_context* c);
-// Same contract as zgemm() for descriptors with KB >= 1; FP64 in, FP64 out.
-int split_zgemm(SplitGemm* e, const ZgemmDesc& d, int slices, cudaStream_t st);
+// Same contract as zgemm() for descriptors with KB >= 1; FP64 in, FP64 out.  keep_b: the caller has
+// run no other GEMM on this engine since one with the same B operand (descriptor and contents) and slice
+// count, so its slices and exponents are used again.
+int split_zgemm(SplitGemm* e, const ZgemmDesc& d, int slices, cudaStream_t st, bool keep_b = false);
 // Same as split_zgemm, recording the row maxima of C as described by mx (alpha = 1, beta = 0).
 int split_zgemm_rowmax(SplitGemm* e, const ZgemmDesc& d, int slices, const SplitRowMax& mx, cudaStream_t st);
 // split_zgemm with operand exponents given (ea [batch][rows_a_pad], eb [batch][N], as
