@@ -285,7 +285,7 @@ std::vector<const void*> gg_context::buffer_signature() const {
   std::vector<const void*> v = {V,       V_owned.p, Uk.p,      Uq.p,    k_f2r_d.p,   k_tr_d.p,   Ttn.p,
                                 Tnt_fold.p, x2c_in.p, x2c_out.p, G_in.p, Sigma_out.p, Gf.p,       Gtmp.p,
                                 Vbuf.p,  G1buf.p,   scratchA.p, scratchB.p, P0buf.p, Pw.p,     Afac.p,
-                                Wt.p,    Wrot.p,    gemm_work.p, hf_D.p,  hf_F.p,      hf_c.p,     hf_J.p,
+                                Wt.p,    Wrot.p,    gemm_work.p, hf_D.p,  hf_F.p,      hf_c.p,     hf_J.p,  hf_S.p,
                                 info.p,  piv.p,     idx_i.p,   pos_d.p,  op_d.p,      gw_err.p,   gw_tables.get(),
                                 p0_ea.p, p0_eb.p,    lu_inv.p};
   split_buffers(split, v);
@@ -528,63 +528,19 @@ int gg_hf_fock(gg_context* c, const double* dm, const double* S_k, double madelu
     if (!dm || !S_k || !F_out) throw Error(GG_ERR_ARG, "hf: NULL buffer");
     const auto& s = c->sh;
     double2* fout = nullptr;
-    double2* din = hf_upload(c, dm, &fout);
+    const double2* din = hf_upload(c, dm, &fout);
+    c->hf_S.upload((const double2*)S_k, (size_t)s.ink * spin_elems(c), c->stream);
     hf_exchange(c, din, fout, c->stream);
     hf_direct(c, fout, c->stream);
-    const size_t m = c->x2c ? 2 * (size_t)s.nao : (size_t)s.nao, mm = m * m;
-    const size_t count = (size_t)s.ink * spin_elems(c);
-    std::vector<double2> F(count);
-    hf_download(c, fout, reinterpret_cast<double*>(F.data()));
-    // Ewald on the host: F -= c * madelung * S D S per (s, IBZ k), c = 0.5 (ns = 1) or 1
-    // (hf_gpu_kernel.cpp:188-201).  X2C: per spin block with the AO overlap S_aa on both
-    // sides and c = 1; the ba block gets the adjoint of the ab term (hf_gpu_kernel.cpp:311-323)
-    const double2* S = (const double2*)S_k;
-    const double2* D = (const double2*)dm;
-    const int n = s.nao;
-    auto sds = [&](const double2* Sb, size_t sld, const double2* Db, size_t dld, double2* out) {
-      std::vector<double2> tmp((size_t)n * n);
-      for (int i = 0; i < n; ++i)
-        for (int j = 0; j < n; ++j) {
-          double2 acc = make_double2(0, 0);
-          for (int a = 0; a < n; ++a) acc = cadd(acc, cmul(Sb[i * sld + a], Db[a * dld + j]));
-          tmp[(size_t)i * n + j] = acc;
-        }
-      for (int i = 0; i < n; ++i)
-        for (int j = 0; j < n; ++j) {
-          double2 acc = make_double2(0, 0);
-          for (int a = 0; a < n; ++a) acc = cadd(acc, cmul(tmp[(size_t)i * n + a], Sb[a * sld + j]));
-          out[(size_t)i * n + j] = acc;
-        }
-    };
-    std::vector<double2> E((size_t)n * n);
-    if (!c->x2c) {
-      const double pre = (s.ns == 2 ? 1.0 : 0.5) * madelung;
-      for (size_t b = 0; b < (size_t)s.ns * s.ink; ++b) {
-        sds(S + b * mm, m, D + b * mm, m, E.data());
-        for (size_t e = 0; e < mm; ++e) F[b * mm + e] = csub(F[b * mm + e], cscale(E[e], pre));
-      }
-    } else {
-      for (size_t k = 0; k < (size_t)s.ink; ++k) {
-        const double2* Sk = S + k * mm;  // S_aa block at (0, 0), leading dimension 2 nao
-        double2* Fk = F.data() + k * mm;
-        const int blocks[3][2] = {{0, 0}, {1, 1}, {0, 1}};
-        for (auto& bl : blocks) {
-          const int a = bl[0], b = bl[1];
-          sds(Sk, m, D + k * mm + (size_t)a * n * m + (size_t)b * n, m, E.data());
-          for (int i = 0; i < n; ++i)
-            for (int j = 0; j < n; ++j) {
-              const double2 v = cscale(E[(size_t)i * n + j], madelung);
-              double2& f = Fk[(size_t)(a * n + i) * m + b * n + j];
-              f = csub(f, v);
-              if (a != b) {
-                double2& g = Fk[(size_t)(n + j) * m + i];
-                g = csub(g, make_double2(v.x, -v.y));
-              }
-            }
-        }
-      }
-    }
-    std::memcpy(F_out, F.data(), count * sizeof(double2));
+    // Ewald: F -= f madelung S D S per (s, IBZ k), f = 0.5 (ns = 1) or 1 (hf_gpu_kernel.cpp:188-201).  X2C: per spin
+    // block with the AO overlap S_aa on both sides and f = 1; the ba block is the adjoint of the ab
+    // one when the blocks are merged (hf_gpu_kernel.cpp:311-323)
+    const long n = s.nao, nn = n * n;
+    if (c->x2c)
+      hf_ewald(c, c->hf_S.p, 2 * s.nao, 0, 4 * nn, din, 3, madelung, fout, c->stream);
+    else
+      hf_ewald(c, c->hf_S.p, s.nao, s.ink * nn, nn, din, s.ns, (s.ns == 2 ? 1.0 : 0.5) * madelung, fout, c->stream);
+    hf_download(c, fout, F_out);
   });
 }
 

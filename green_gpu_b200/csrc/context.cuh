@@ -99,7 +99,7 @@ struct gg_context {
 
   // work buffers
   gg::DevBuf<double2> G_in, Sigma_out, Gf, Gtmp, Vbuf, G1buf, scratchA, scratchB, P0buf, Pw, Afac, Wt, Wrot,
-      gemm_work, hf_D, hf_F, hf_c, hf_J, lu_inv;
+      gemm_work, hf_D, hf_F, hf_c, hf_J, hf_S, lu_inv;
   gg::DevBuf<int> info, piv, idx_i;
   // split precision: exponents of the P0 main contraction's operand rows / columns, recorded
   // by the operand builds' epilogues
@@ -120,6 +120,7 @@ struct gg_context {
   // tables of one GW build (pair positions and ops, G block indices), built on the first build
   // after the symmetry, k-pairs or spin layout changed
   std::shared_ptr<void> gw_tables;
+  std::shared_ptr<void> hf_tables;  // pair tables of the HF calls
   // graph mode: the first build runs eagerly, the second is captured into a CUDA graph that
   // later builds replay while inputs, buffers and settings match (any setter drops it)
   bool graph_mode = false;
@@ -146,6 +147,7 @@ struct gg_context {
   std::vector<const void*> buffer_signature() const;
   void invalidate() {
     gw_tables.reset();
+    hf_tables.reset();
     drop_graph();
   }
 

@@ -750,6 +750,38 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
 }
 
 // ---------------------------------------------------------------------------------------
+namespace {
+
+// tables of the HF calls, kept in the context: the pairs (k_ibz, k2) of the exchange (k2 fastest), the diagonal
+// pairs (k, k) of the Hartree term, and the full-BZ index of every irreducible k
+struct HfTables {
+  PairTable pairs, diag;
+  IntTable k_r2f;
+};
+
+const HfTables& hf_tables(gg_context* c) {
+  if (!c->hf_tables) {
+    auto tab = std::make_shared<HfTables>();
+    const auto& s = c->sh;
+    std::vector<int> a, b, r;
+    for (int kr = 0; kr < s.ink; ++kr)
+      for (int k2 = 0; k2 < s.nk; ++k2) {
+        a.push_back((int)c->k_r2f[kr]);
+        b.push_back(k2);
+      }
+    tab->pairs.build(c, a, b);
+    a.clear();
+    for (int k = 0; k < s.nk; ++k) a.push_back(k);
+    tab->diag.build(c, a, a);
+    for (int kr = 0; kr < s.ink; ++kr) r.push_back((int)c->k_r2f[kr]);
+    tab->k_r2f.build(r);
+    c->hf_tables = tab;
+  }
+  return *std::static_pointer_cast<HfTables>(c->hf_tables);
+}
+
+}  // namespace
+
 // HF exchange K_s(k) = pref/nk sum_k2 sum_Q V^Q(k,k2) D_s(k2) V^Q(k,k2)^+ (cuhf_utils.cu:108-134)
 void hf_exchange(gg_context* c, const double2* dm_dev, double2* K_dev, cudaStream_t st) {
   if (!c->has_sym || !c->has_kpairs || !c->V)
@@ -762,37 +794,38 @@ void hf_exchange(gg_context* c, const double2* dm_dev, double2* K_dev, cudaStrea
   // unfolded density D[k][s][i][j]
   double2* D = c->hf_D.ensure((size_t)nk * ns * nn);
   c->Gtmp.ensure((size_t)nk * ns * nn);
-  const size_t room = (size_t)(0.4 * (double)free_bytes()) / (2 * Nnn * sizeof(double2));
-  const int kc = (int)std::max<size_t>(1, std::min<size_t>(nk, room));
-  double2* Vb = c->Vbuf.ensure((size_t)kc * Nnn);
-  double2* X = c->scratchA.ensure((size_t)kc * Nnn);
-  double2* work = c->gemm_work.ensure((size_t)1 << 22);
-  PairTable pairs;
-  {
-    std::vector<int> a, b;
-    for (int kr = 0; kr < s.ink; ++kr)
-      for (int k2 = 0; k2 < nk; ++k2) {
-        a.push_back((int)c->k_r2f[kr]);
-        b.push_back(k2);
-      }
-    pairs.build(c, a, b);
+  // pairs per step: all k2 of as many irreducible k as 256 MB of integrals hold (at least one, so that
+  // a small system takes few launches), or k2 in chunks when the device has less room than that
+  const int krc = (int)std::max<long>(1, std::min<long>(s.ink, (256L << 20) / ((long)nk * Nnn * (long)sizeof(double2))));
+  int kc = nk, kg = krc;  // k2 and irreducible k per step
+  const size_t want = (size_t)krc * nk * Nnn;
+  if (c->Vbuf.n < want || c->scratchA.n < want) {
+    const size_t room = (size_t)(0.4 * (double)free_bytes()) / (2 * Nnn * sizeof(double2));
+    kc = (int)std::max<size_t>(1, std::min<size_t>(nk, room));
+    if (room < (size_t)krc * nk) kg = 1;
   }
+  double2* Vb = c->Vbuf.ensure((size_t)kg * kc * Nnn);
+  double2* X = c->scratchA.ensure((size_t)kg * kc * Nnn);
+  double2* work = c->gemm_work.ensure((size_t)1 << 22);
+  const HfTables& tab = hf_tables(c);
   unfold_matrices(c, dm_dev, 1, ns, D, st);  // layout [k][s][n][n]
   GG_CUDA(cudaMemsetAsync(K_dev, 0, sizeof(double2) * (size_t)ns * s.ink * nn, st));
   const double pref = ns == 1 ? -0.5 : -1.0;
-  for (int kr = 0; kr < s.ink; ++kr) {
+  for (int kr = 0; kr < s.ink; kr += kg) {
+    const int rn = std::min(kg, s.ink - kr);
     for (int k0 = 0; k0 < nk; k0 += kc) {
       const int kn = std::min(kc, nk - k0);
-      pairs.gather(c, (size_t)kr * nk + k0, kn, Vb, st);
+      tab.pairs.gather(c, (size_t)kr * nk + k0, rn * kn, Vb, st);
       ++c->launches;
       for (int sp = 0; sp < ns; ++sp) {
-        // X[kk][Q][j][c] = sum_a V[kk][Q][j][a] D[k2][sp][a][c]   (cuhf_utils.cu:118)
+        // X[r][kk][Q][j][c] = sum_a V[r][kk][Q][j][a] D[k2][sp][a][c]   (cuhf_utils.cu:118)
         ZgemmDesc d;
         d.M = N * n; d.N = n; d.K = n;
         d.A = Vb; d.a_m.lo = n; d.a_k = 1;
         d.B = D + ((long)k0 * ns + sp) * nn; d.b_k = n; d.b_n.lo = 1;
         d.C = X; d.c_m.lo = n; d.c_n.lo = 1;
         d.nb0 = kn; d.a_b0 = Nnn; d.b_b0 = (long)ns * nn; d.c_b0 = Nnn;
+        d.nb1 = rn; d.a_b1 = kn * Nnn; d.c_b1 = kn * Nnn;
         d.work = work; d.work_elems = (long)c->gemm_work.n;
         c->launches += zgemm(d, st);
         // K[sp][kr][j][i] += pref/nk sum_{kk,Q} sum_c X[kk][Q][j][c] conj(V[kk][Q][i][c])  (:127-131)
@@ -802,6 +835,7 @@ void hf_exchange(gg_context* c, const double2* dm_dev, double2* K_dev, cudaStrea
         e.A = X; e.a_m.lo = n; e.a_k = 1; e.a_kb = nn;
         e.B = Vb; e.b_k = 1; e.b_n.lo = n; e.b_kb = nn; e.conjB = 1;
         e.C = K_dev + ((long)sp * s.ink + kr) * nn; e.c_m.lo = n; e.c_n.lo = 1;
+        e.nb0 = rn; e.a_b0 = kn * Nnn; e.b_b0 = kn * Nnn; e.c_b0 = nn;
         e.alpha = make_double2(pref / nk, 0.0);
         e.beta = make_double2(1.0, 0.0);
         e.work = work; e.work_elems = (long)c->gemm_work.n;
@@ -816,41 +850,39 @@ void hf_exchange(gg_context* c, const double2* dm_dev, double2* K_dev, cudaStrea
 }
 
 // Hartree (direct) term J(k) = sum_Q c_Q V^Q(k,k), c_Q = 1/nk sum_{s,k'} Tr(V^Q(k',k') D_s(k'))
-// (hf_gpu_kernel.cpp:141-186).  Uses the unfolded density left in c->hf_D by hf_exchange.
+// (hf_gpu_kernel.cpp:141-186), added to F.  Uses the unfolded density left in c->hf_D by hf_exchange.
 void hf_direct(gg_context* c, double2* F_dev, cudaStream_t st) {
   const auto& s = c->sh;
   // X2C: the density of the aa and bb blocks, J added to both (hf_gpu_kernel.cpp:269-309)
-  const int n = s.nao, N = s.NQ, nk = s.nk, ns = hf_spins(c), nsj = c->x2c ? 2 : ns;
-  const long nn = (long)n * n, Nnn = (long)N * nn;
-  double2* cq = c->hf_c.ensure(N);
-  GG_CUDA(cudaMemsetAsync(cq, 0, sizeof(double2) * N, st));
-  const int kc = (int)std::max<size_t>(1, std::min<size_t>(nk, c->Vbuf.n / Nnn));
-  double2* Vb = c->Vbuf.ensure((size_t)kc * Nnn);
-  double2* Dk = c->hf_J.ensure((size_t)kc * nn);
-  PairTable diag;
-  IntTable didx;
-  {
-    std::vector<int> a(nk), v;
-    for (int k = 0; k < nk; ++k) a[k] = k;
-    diag.build(c, a, a);
-    for (int sp = 0; sp < ns; ++sp)
-      for (int k = 0; k < nk; ++k) v.push_back(k * ns + sp);
-    didx.build(v);
-  }
-  for (int k0 = 0; k0 < nk; k0 += kc) {
-    const int kn = std::min(kc, nk - k0);
-    diag.gather(c, k0, kn, Vb, st);
-    for (int sp = 0; sp < nsj; ++sp) {
-      launch_gather_blocks(c->hf_D.p, didx.d.p + (size_t)sp * nk + k0, kn, nn, nn, Dk, st);
-      launch_hartree_coeff(Vb, Dk, kn, N, n, 1.0 / nk, cq, st);
-    }
-  }
-  double2* J = c->scratchB.ensure((size_t)nn);
-  for (int kr = 0; kr < s.ink; ++kr) {
-    diag.gather(c, (size_t)c->k_r2f[kr], 1, Vb, st);
-    launch_hartree_apply(Vb, cq, N, n, J, st);
-    for (int sp = 0; sp < nsj; ++sp) launch_axpy(F_dev + ((long)sp * s.ink + kr) * nn, J, nn, st);
-  }
+  const int ns = hf_spins(c), nsj = c->x2c ? 2 : ns;
+  double2* cq = c->hf_c.ensure((size_t)(s.nk + 1) * s.NQ);
+  const HfTables& tab = hf_tables(c);
+  launch_hartree_coeff(c->V, tab.diag.pos.p, tab.diag.op.p, c->hf_D.p, s.nk, s.NQ, s.nao, ns, nsj, 1.0 / s.nk, cq, st);
+  launch_hartree_apply(c->V, tab.diag.pos.p, tab.diag.op.p, tab.k_r2f.d.p, cq, s.ink, s.NQ, s.nao, nsj, F_dev, st);
+}
+
+// Ewald term F -= pre S D S per (block, irreducible k); S [.][ink] matrices with row stride ldS (X2C: the aa
+// block of the spinor overlap on both sides), D and F blocks [nblk][ink][n][n]
+// (hf_gpu_kernel.cpp:188-201, 311-323)
+void hf_ewald(gg_context* c, const double2* S, int ldS, long s_blk, long s_k, const double2* D, int nblk, double pre,
+              double2* F_dev, cudaStream_t st) {
+  const int n = c->sh.nao, ink = c->sh.ink;
+  const long nn = (long)n * n;
+  ZgemmDesc d;
+  d.M = n; d.N = n; d.K = n;
+  d.A = S; d.a_m.lo = ldS; d.a_k = 1;
+  d.B = D; d.b_k = n; d.b_n.lo = 1;
+  d.C = c->hf_J.ensure((size_t)nblk * ink * nn); d.c_m.lo = n; d.c_n.lo = 1;
+  d.nb0 = ink; d.a_b0 = s_k; d.b_b0 = nn; d.c_b0 = nn;
+  d.nb1 = nblk; d.a_b1 = s_blk; d.b_b1 = ink * nn; d.c_b1 = ink * nn;
+  zgemm(d, st);
+  ZgemmDesc e = d;
+  e.A = d.C; e.a_m.lo = n; e.a_b0 = nn; e.a_b1 = ink * nn;
+  e.B = S; e.b_k = ldS; e.b_b0 = s_k; e.b_b1 = s_blk;
+  e.C = F_dev;
+  e.alpha = make_double2(-pre, 0.0);
+  e.beta = make_double2(1.0, 0.0);
+  zgemm(e, st);
 }
 
 }  // namespace gg

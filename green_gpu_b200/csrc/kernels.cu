@@ -96,11 +96,6 @@ __global__ void transpose_blocks_kernel(const double2* __restrict__ in, int n, i
   }
 }
 
-__global__ void axpy_kernel(double2* y, const double2* x, long n) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-    y[i] = cadd(y[i], x[i]);
-}
-
 __global__ void scale_kernel(double2* X, long n, double s) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
     X[i] = cscale(X[i], s);
@@ -111,37 +106,68 @@ inline unsigned grid_for(long n, int tpb = TPB) {
   return (unsigned)std::max(1L, std::min(b, 148L * 32));
 }
 
-__global__ void hartree_coeff_kernel(const double2* __restrict__ V, const double2* __restrict__ D, int npairs, int NQ,
-                                     int n, double scale, double2* c) {
-  // one block per Q; c[Q] += scale * sum_p sum_ab V[p][Q][a][b] D[p][b][a]
-  __shared__ double2 red[TPB];
-  const int Q = blockIdx.x;
-  const long nn = (long)n * n;
+// One CTA per (Q, k): cp[k][Q] = sum_{s < nsj} Tr(V^Q(k,k) D_s(k)), V(k,k) = op(stored).  The stored
+// matrix is read in its own order, so that the pass streams the integrals once (HBM-bound); the
+// element of D that meets S[r][c] is D[c][r], or D[r][c] under a transpose.
+__global__ void __launch_bounds__(128) hartree_coeff_kernel(const double2* __restrict__ S, const int64_t* __restrict__ pos,
+                                                            const int* __restrict__ op, const double2* __restrict__ D, int NQ,
+                                                            int n, int ns, int nsj, double2* __restrict__ cp) {
+  __shared__ double2 red[4];
+  const int Q = blockIdx.x, k = blockIdx.y;
+  const int nn = n * n;
+  const double2* v = S + (pos[k] * NQ + Q) * (long)nn;
+  const double2* d = D + (long)k * ns * nn;
+  const bool cj = op[k] & 1, tr = (op[k] >> 1) & 1;
   double2 acc = make_double2(0, 0);
-  for (int p = 0; p < npairs; ++p) {
-    const double2* v = V + ((long)p * NQ + Q) * nn;
-    const double2* d = D + (long)p * nn;
-    for (long e = threadIdx.x; e < nn; e += TPB) {
-      int a = (int)(e / n), b = (int)(e % n);
-      acc = cadd(acc, cmul(v[e], d[(long)b * n + a]));
-    }
+  for (int e = threadIdx.x; e < nn; e += 128) {
+    const int r = e / n, c = e - r * n;
+    double2 x = v[e];
+    if (cj) x.y = -x.y;
+    for (int s = 0; s < nsj; ++s) acc = cadd(acc, cmul(x, d[(long)s * nn + (tr ? e : c * n + r)]));
   }
-  red[threadIdx.x] = acc;
+  for (int o = 16; o > 0; o >>= 1) {
+    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+  }
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
-  for (int s = TPB / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = cadd(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) c[Q] = cadd(c[Q], cscale(red[0], scale));
+  if (threadIdx.x == 0) cp[(long)k * NQ + Q] = cadd(cadd(red[0], red[1]), cadd(red[2], red[3]));
 }
 
-__global__ void hartree_apply_kernel(const double2* __restrict__ V, const double2* __restrict__ c, int NQ, int n,
-                                     double2* J) {
-  const long nn = (long)n * n;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < nn; e += (long)gridDim.x * blockDim.x) {
-    double2 acc = make_double2(0, 0);
-    for (int Q = 0; Q < NQ; ++Q) acc = cadd(acc, cmul(c[Q], V[(long)Q * nn + e]));
-    J[e] = acc;
+// c[Q] = scale sum_k cp[k][Q], in the order of k
+__global__ void hartree_sum_kernel(const double2* __restrict__ cp, int nk, int NQ, double scale, double2* __restrict__ c) {
+  const int Q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (Q >= NQ) return;
+  double2 acc = make_double2(0, 0);
+  for (int k = 0; k < nk; ++k) acc = cadd(acc, cp[(long)k * NQ + Q]);
+  c[Q] = cscale(acc, scale);
+}
+
+// F[s][kr] += op(sum_Q c[Q] S[Q]) for s < nsj: one CTA per (32 elements, kr), eight warps sharing the Q
+__global__ void __launch_bounds__(256) hartree_apply_kernel(const double2* __restrict__ S, const int64_t* __restrict__ pos,
+                                                            const int* __restrict__ op, const int* __restrict__ k_r2f,
+                                                            const double2* __restrict__ c, int ink, int NQ, int n, int nsj,
+                                                            double2* __restrict__ F) {
+  __shared__ double2 red[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int kr = blockIdx.y, k = k_r2f[kr], nn = n * n, e = blockIdx.x * 32 + lane;
+  const bool cj = op[k] & 1, tr = (op[k] >> 1) & 1;
+  const double2* v = S + pos[k] * NQ * (long)nn;
+  double2 acc = make_double2(0, 0);
+  if (e < nn)
+    for (int Q = w; Q < NQ; Q += 8) {
+      double2 x = v[(long)Q * nn + e];
+      if (cj) x.y = -x.y;
+      acc = cadd(acc, cmul(c[Q], x));
+    }
+  red[w][lane] = acc;
+  __syncthreads();
+  if (w != 0 || e >= nn) return;
+  for (int i = 1; i < 8; ++i) acc = cadd(acc, red[i][lane]);
+  const int r = e / n, q = e - r * n, o = tr ? q * n + r : e;
+  for (int s = 0; s < nsj; ++s) {
+    double2* f = F + ((long)s * ink + kr) * nn + o;
+    *f = cadd(*f, acc);
   }
 }
 
@@ -250,11 +276,6 @@ void launch_transpose_blocks(const double2* in, long nblocks, int n, double2* ou
   GG_CHECK_LAUNCH();
 }
 
-void launch_axpy(double2* y, const double2* x, long n, cudaStream_t st) {
-  axpy_kernel<<<grid_for(n), TPB, 0, st>>>(y, x, n);
-  GG_CHECK_LAUNCH();
-}
-
 void launch_scale(double2* X, long n, double s, cudaStream_t st) {
   scale_kernel<<<grid_for(n), TPB, 0, st>>>(X, n, s);
   GG_CHECK_LAUNCH();
@@ -264,14 +285,17 @@ void launch_fill_zero(double2* X, long n, cudaStream_t st) {
   GG_CUDA(cudaMemsetAsync(X, 0, sizeof(double2) * n, st));
 }
 
-void launch_hartree_coeff(const double2* V, const double2* D, int npairs, int NQ, int n, double scale, double2* c,
-                          cudaStream_t st) {
-  hartree_coeff_kernel<<<NQ, TPB, 0, st>>>(V, D, npairs, NQ, n, scale, c);
+void launch_hartree_coeff(const double2* S, const int64_t* pos_d, const int* op_d, const double2* D, int nk, int NQ, int n,
+                          int ns, int nsj, double scale, double2* c, cudaStream_t st) {
+  hartree_coeff_kernel<<<dim3(NQ, nk), 128, 0, st>>>(S, pos_d, op_d, D, NQ, n, ns, nsj, c + NQ);
+  GG_CHECK_LAUNCH();
+  hartree_sum_kernel<<<ceil_div(NQ, 64), 64, 0, st>>>(c + NQ, nk, NQ, scale, c);
   GG_CHECK_LAUNCH();
 }
 
-void launch_hartree_apply(const double2* V, const double2* c, int NQ, int n, double2* J, cudaStream_t st) {
-  hartree_apply_kernel<<<grid_for((long)n * n), TPB, 0, st>>>(V, c, NQ, n, J);
+void launch_hartree_apply(const double2* S, const int64_t* pos_d, const int* op_d, const int* k_r2f_d, const double2* c,
+                          int ink, int NQ, int n, int nsj, double2* F, cudaStream_t st) {
+  hartree_apply_kernel<<<dim3(ceil_div((long)n * n, 32), ink), 256, 0, st>>>(S, pos_d, op_d, k_r2f_d, c, ink, NQ, n, nsj, F);
   GG_CHECK_LAUNCH();
 }
 

@@ -21,8 +21,6 @@ void launch_conj_where(double2* X, const int* tr_d, int nk, long per_k, cudaStre
 // gather blocks: out[p][e] = src[idx[p] * src_stride + e] for e < elems
 void launch_gather_blocks(const double2* src, const int* idx_d, int nblocks, long elems, long src_stride,
                           double2* out, cudaStream_t st);
-// y += x (n complex numbers)
-void launch_axpy(double2* y, const double2* x, long n, cudaStream_t st);
 // err[0..2] <- (1, base + i, info[i]) for a failing system i (info != 0), if none is recorded yet
 void launch_info_collect(const int* info, int count, int base, int* err, cudaStream_t st);
 
@@ -55,10 +53,12 @@ int launch_dyson(double2* P, double2* A, double2* li, int* info, int nsys, int N
 // Hermitian symmetrisation only (cuda_common.cu:249-281), nsys matrices in place.
 void launch_hermitian_symmetrize(double2* P, int nsys, int N, cudaStream_t st);
 
-// Hartree coefficients: c[Q] += scale * sum_{ab} V[p][Q][a][b] D[p][b][a] over p (pairs).
-void launch_hartree_coeff(const double2* V, const double2* D, int npairs, int NQ, int n, double scale, double2* c,
-                          cudaStream_t st);
-// J[i][j] = sum_Q c[Q] V[Q][i][j]
-void launch_hartree_apply(const double2* V, const double2* c, int NQ, int n, double2* J, cudaStream_t st);
+// Hartree term on the stored integrals (pos / op of the diagonal pairs (k, k)):
+// c[Q] = scale sum_k sum_{s < nsj} Tr(V^Q(k,k) D[k][s]) (c holds (nk + 1) NQ elements, the partial sums of
+// every k after the result), F[s][kr] += sum_Q c[Q] V^Q(k,k) for s < nsj, k = k_r2f[kr].
+void launch_hartree_coeff(const double2* S, const int64_t* pos_d, const int* op_d, const double2* D, int nk, int NQ, int n,
+                          int ns, int nsj, double scale, double2* c, cudaStream_t st);
+void launch_hartree_apply(const double2* S, const int64_t* pos_d, const int* op_d, const int* k_r2f_d, const double2* c,
+                          int ink, int NQ, int n, int nsj, double2* F, cudaStream_t st);
 
 }  // namespace gg

@@ -9,38 +9,44 @@
 namespace gg {
 namespace {
 
-__global__ void zgemm_reduce(ZgemmDesc d) {
-  const long batch_count = (long)d.nb0 * d.nb1 * d.nb2;
-  const long mn = (long)d.M * d.N;
-  const long total = batch_count * mn;
-  const bool use_beta = d.beta.x != 0.0 || d.beta.y != 0.0;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const long batch = i / mn;
-    const long e = i % mn;
-    const int m = (int)(e / d.N);
-    const int n = (int)(e % d.N);
-    double2 acc = make_double2(0.0, 0.0);
-    // partial sums in order, eight loads in flight
+// C = alpha sum_s work[s] + beta C.  SL threads share the partial sums of an element (consecutive runs,
+// then combined in order), eight loads in flight each, so that hundreds of partial sums of a small
+// output are not one chain of loads.
+template <int SL>
+__global__ void __launch_bounds__(256) zgemm_reduce(ZgemmDesc d) {
+  __shared__ double2 part[SL > 1 ? SL : 1][SL > 1 ? 256 / SL : 1];
+  const long mn = (long)d.M * d.N, total = (long)d.nb0 * d.nb1 * d.nb2 * mn;
+  const int lane = threadIdx.x % (256 / SL), sl = threadIdx.x / (256 / SL);
+  const long i = blockIdx.x * (long)(256 / SL) + lane;
+  double2 acc = make_double2(0.0, 0.0);
+  if (i < total) {
     const double2* w = d.work + i;
-    int s = 0;
-    for (; s + 8 <= d.splits; s += 8) {
+    int s = d.splits * sl / SL;
+    const int end = d.splits * (sl + 1) / SL;
+    for (; s + 8 <= end; s += 8) {
       double2 p[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) p[j] = w[(s + j) * total];
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc = cadd(acc, p[j]);
     }
-    for (; s < d.splits; ++s) acc = cadd(acc, w[s * total]);
-    const int b0 = (int)(batch % d.nb0);
-    const int b1 = (int)((batch / d.nb0) % d.nb1);
-    const int b2 = (int)(batch / ((long)d.nb0 * d.nb1));
-    double2* c = d.C + b0 * d.c_b0 + b1 * d.c_b1 + b2 * d.c_b2 + d.c_m(m) + d.c_n(n);
-    double2 v = cmul(d.alpha, acc);
-    if (use_beta) v = cadd(v, cmul(d.beta, *c));
-    *c = v;
+    for (; s < end; ++s) acc = cadd(acc, w[s * total]);
   }
+  if constexpr (SL > 1) {
+    part[sl][lane] = acc;
+    __syncthreads();
+    if (sl != 0) return;
+    for (int j = 1; j < SL; ++j) acc = cadd(acc, part[j][lane]);
+  }
+  if (i >= total) return;
+  const long batch = i / mn, e = i % mn;
+  const int m = (int)(e / d.N), n = (int)(e % d.N);
+  const int b0 = (int)(batch % d.nb0), b1 = (int)((batch / d.nb0) % d.nb1), b2 = (int)(batch / ((long)d.nb0 * d.nb1));
+  double2* c = d.C + b0 * d.c_b0 + b1 * d.c_b1 + b2 * d.c_b2 + d.c_m(m) + d.c_n(n);
+  double2 v = cmul(d.alpha, acc);
+  if (d.beta.x != 0.0 || d.beta.y != 0.0) v = cadd(v, cmul(d.beta, *c));
+  *c = v;
 }
-
 
 // Tile shape and split-K factor of a descriptor.
 struct ZChoice {
@@ -60,7 +66,7 @@ struct ZChoice {
 //   l2     operand tiles arrive at about 40 bytes per cycle and SM.
 // Splitting the reduction multiplies the tiles and adds a launch and the pass over the partial sums.
 ZChoice choose(const ZgemmDesc& d, long batch, long groups, int sms) {
-  static const int kSplits[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 48, 64};
+  static const int kSplits[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 48, 64, 96, 128, 192, 256, 384, 512};
   const ZShape* const table = d.gauss ? kZShape3 : kZShape;
   const int count = d.gauss ? kZShapes3 : kZShapes;
   const double prods = d.gauss ? 3.0 : 4.0;
@@ -84,7 +90,7 @@ ZChoice choose(const ZgemmDesc& d, long batch, long groups, int sms) {
       const double chain = waves * (g * group + 150.0 * t88 + 9000.0);
       const double l2 = per_sm * (s.bm + s.bn) * g * 64.0 / 40.0;
       double cost = std::max(std::max(pipe, chain), l2);
-      if (sp > 1) cost += 6000.0 + 250.0 * sp + out * (sp + 1) * 16.0 / 3000.0;
+      if (sp > 1) cost += 7000.0 + 100.0 * std::min(sp, 64) + out * (sp + 1) * 16.0 / 3000.0;
       if (!have || cost < best_cost) {
         have = true;
         best_cost = cost;
@@ -147,9 +153,10 @@ int zgemm(const ZgemmDesc& d0, cudaStream_t stream) {
   int launches = 1;
   if (d.splits > 1) {
     const long total = (long)d.M * d.N * batch;
-    const int threads = 256;
-    const long nblk = std::min<long>((total + threads - 1) / threads, 65535L * 8);
-    zgemm_reduce<<<(unsigned)nblk, threads, 0, stream>>>(d);
+    if (d.splits > 32)
+      zgemm_reduce<8><<<(unsigned)((total + 31) / 32), 256, 0, stream>>>(d);
+    else
+      zgemm_reduce<1><<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(d);
     GG_CHECK_LAUNCH();
     ++launches;
   }
