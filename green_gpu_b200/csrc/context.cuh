@@ -133,6 +133,7 @@ struct gg_context {
   // device addresses of every work buffer when the graph was captured: an entry point that
   // grows a shared buffer (HF, unfold, zgemm) reallocates it, and the graph is then rebuilt
   std::vector<const void*> graph_sig;
+  gg::DevBuf<int> gw_flag;  // nonzero: this build's G is Hermitian
   gg::DevBuf<int> gw_err;  // [0] failed, [1] system index (q position x nw_b + Omega), [2] info
   int plan_qc = 0, plan_kc = 0, plan_tb = 0;  // plan of the eager build, reused by the capture
 

@@ -101,6 +101,64 @@ __global__ void scale_kernel(double2* X, long n, double s) {
     X[i] = cscale(X[i], s);
 }
 
+// One CTA per matrix (blockIdx.x = (t * ns + s) * ink + k): clears *flag unless G[t][s][k] and G[t][s'][k]^H agree
+// within 2^-46 of the largest element of either, s' = s or, with `swap` (X2C spin blocks), 0, 1, 3, 2
+__global__ void __launch_bounds__(128) hermitian_check_kernel(const double2* __restrict__ G, int ns, int ink, int n, int swap,
+                                                              int* flag) {
+  __shared__ double red[2][4];
+  const long nn = (long)n * n;
+  const long b = blockIdx.x;
+  const int s = (int)((b / ink) % ns), p = swap && s >= 2 ? 5 - s : s;
+  const double2* X = G + b * nn;
+  const double2* Y = X + (long)(p - s) * ink * nn;
+  double big = 0.0, off = 0.0;
+  bool bad = false;
+  for (int e = threadIdx.x; e < nn; e += 128) {
+    const int i = e / n, j = e - i * n;
+    const double2 x = X[e], y = Y[(long)j * n + i];
+    const double m = fmax(fmax(fabs(x.x), fabs(x.y)), fmax(fabs(y.x), fabs(y.y)));
+    const double o = fmax(fabs(x.x - y.x), fabs(x.y + y.y));
+    bad = bad || !(o <= 1e300);  // NaN and infinities
+    big = fmax(big, m);
+    off = fmax(off, o);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+    off = fmax(off, __shfl_xor_sync(0xffffffffu, off, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = big;
+    red[1][threadIdx.x >> 5] = off;
+  }
+  const int any_bad = __syncthreads_or(bad);
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 4; ++w) {
+      big = fmax(big, red[0][w]);
+      off = fmax(off, red[1][w]);
+    }
+    if (any_bad || off > 0x1p-46 * big) *flag = 0;
+  }
+}
+
+// where *flag: X[b][i][j] = conj(X[b][j][i]) above the diagonal and a real diagonal; one 32 x 32 tile pair per CTA
+__global__ void __launch_bounds__(TPB) mirror_lower_kernel(double2* X, int n, const int* flag) {
+  __shared__ double2 s[32][33];
+  if (!*flag) return;
+  int ti = 0, tj = blockIdx.y;
+  while (tj > ti) tj -= ++ti;  // tile row ti >= tile column tj
+  double2* M = X + blockIdx.x * (long)n * n;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int r = ty; r < 32; r += 8) {
+    const int i = ti * 32 + r, j = tj * 32 + tx;
+    if (i < n && j < n) s[r][tx] = M[(long)i * n + j];
+  }
+  __syncthreads();
+  for (int r = ty; r < 32; r += 8) {
+    const int i = tj * 32 + r, j = ti * 32 + tx;
+    if (i < n && j < n && j >= i) M[(long)i * n + j] = i == j ? make_double2(s[r][r].x, 0.0) : cconj(s[tx][r]);
+  }
+}
+
 inline unsigned grid_for(long n, int tpb = TPB) {
   long b = (n + tpb - 1) / tpb;
   return (unsigned)std::max(1L, std::min(b, 148L * 32));
@@ -273,6 +331,18 @@ void launch_transpose_blocks(const double2* in, long nblocks, int n, double2* ou
   if (nblocks > 65535) throw Error(GG_ERR_ARG, "transpose: too many blocks for one launch");
   const int tiles = (n + 31) / 32;
   transpose_blocks_kernel<<<dim3((unsigned)(tiles * tiles), (unsigned)nblocks), dim3(32, 8), 0, st>>>(in, n, tiles, out);
+  GG_CHECK_LAUNCH();
+}
+
+void launch_hermitian_check(const double2* G, int nts, int ns, int ink, int n, int swap, int* flag, cudaStream_t st) {
+  GG_CUDA(cudaMemsetAsync(flag, 1, sizeof(int), st));
+  hermitian_check_kernel<<<nts * ns * ink, 128, 0, st>>>(G, ns, ink, n, swap, flag);
+  GG_CHECK_LAUNCH();
+}
+
+void launch_mirror_lower(double2* X, int nmat, int n, const int* flag, cudaStream_t st) {
+  const int t = ceil_div(n, 32);
+  mirror_lower_kernel<<<dim3(nmat, t * (t + 1) / 2), TPB, 0, st>>>(X, n, flag);
   GG_CHECK_LAUNCH();
 }
 

@@ -41,11 +41,19 @@ __global__ void __launch_bounds__(256) zgemm_reduce(ZgemmDesc d) {
   if (i >= total) return;
   const long batch = i / mn, e = i % mn;
   const int m = (int)(e / d.N), n = (int)(e % d.N);
+  if (d.tri && *d.tri && n > m) return;
   const int b0 = (int)(batch % d.nb0), b1 = (int)((batch / d.nb0) % d.nb1), b2 = (int)(batch / ((long)d.nb0 * d.nb1));
   double2* c = d.C + b0 * d.c_b0 + b1 * d.c_b1 + b2 * d.c_b2 + d.c_m(m) + d.c_n(n);
   double2 v = cmul(d.alpha, acc);
   if (d.beta.x != 0.0 || d.beta.y != 0.0) v = cadd(v, cmul(d.beta, *c));
   *c = v;
+}
+
+// tiles on and below the diagonal of a square product
+int tri_tiles(int tiles_m, int tiles_n, int bm, int bn) {
+  int count = 0;
+  for (int tn = 0; tn < tiles_n; ++tn) count += std::max(0, tiles_m - zfirst_row(tn, bm, bn));
+  return count;
 }
 
 // Tile shape and split-K factor of a descriptor.
@@ -78,7 +86,7 @@ ZChoice choose(const ZgemmDesc& d, long batch, long groups, int sms) {
     const ZShape& s = table[i];
     const int tm = ceil_div(d.M, s.bm), tn = ceil_div(d.N, s.bn);
     if ((d.inplace == 1 && tn > 1) || (d.inplace == 2 && tm > 1)) continue;
-    const double tiles = (double)tm * tn * batch;
+    const double tiles = (double)(d.tri ? tri_tiles(tm, tn, s.bm, s.bn) : tm * tn) * batch;
     const int t88 = s.mt * s.nt;
     const double mma = t88 * prods * 16.0, busy = (0.89 - 0.8 / t88) * (d.gauss ? 0.8 : 1.0);
     const double group = std::max(1.15 * mma + 100.0, 150.0 + 5.0 * (s.bm + s.bn));
@@ -127,6 +135,7 @@ int zgemm(const ZgemmDesc& d0, cudaStream_t stream) {
   ZgemmDesc d = d0;
   if (d.M <= 0 || d.N <= 0 || d.nb0 <= 0 || d.nb1 <= 0 || d.nb2 <= 0) return 0;
   if (d.K < 0 || d.KB < 1) throw Error(GG_ERR_ARG, "zgemm: bad K");
+  if (d.tri && d.M != d.N) throw Error(GG_ERR_INTERNAL, "zgemm: the lower triangle of a product that is not square");
   const long batch = (long)d.nb0 * d.nb1 * d.nb2;
   ZGrid g;
   g.gpb = std::max(1, ceil_div(d.K, 4));
@@ -139,6 +148,7 @@ int zgemm(const ZgemmDesc& d0, cudaStream_t stream) {
   d.splits = ch.splits;
   g.tiles_m = ceil_div(d.M, s.bm);
   g.tiles_n = ceil_div(d.N, s.bn);
+  g.tri_tiles = tri_tiles(g.tiles_m, g.tiles_n, s.bm, s.bn);
   const long items = (long)g.tiles_m * g.tiles_n * d.splits * batch;
   if (items > 0x7fffffffL - 4096 || groups > 0x7fffffffL) throw Error(GG_ERR_ARG, "zgemm: grid too large");
   g.items = (int)items;

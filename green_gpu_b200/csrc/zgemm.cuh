@@ -52,6 +52,9 @@ struct ZgemmDesc {
   // (the same columns, the whole height M is one tile); the operand's tile is read before C's is
   // written and the reduction is not split
   int inplace = 0;
+  // device flag: nonzero restricts a square product to the tiles on and below the diagonal (the elements
+  // above stay undefined; the caller mirrors them)
+  const int* tri = nullptr;
   int splits = 1;            // split-K factor (deterministic: partials + ordered reduction)
   double2* work = nullptr;   // [splits][batch][M][N] when splits > 1
   long work_elems = 0;       // capacity of `work` in complex elements

@@ -41,6 +41,7 @@ constexpr int kZBK = 8;  // reduction elements per stage: two groups of 4
 struct ZGrid {
   int tiles_m, tiles_n;
   int items;            // tiles_m * tiles_n * splits * batch
+  int tri_tiles;        // tiles on and below the diagonal
   int gpb;              // groups of 4 per K-batch
   int groups;           // KB * gpb
   long wrap_a, wrap_b;  // from the last group of a K-batch to the first of the next
@@ -69,12 +70,33 @@ __device__ __forceinline__ void zbar_arrive(int id, int threads) {
   asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// tile row that holds the diagonal of tile column tn: the first one of a lower-triangle product
+__host__ __device__ __forceinline__ int zfirst_row(int tn, int bm, int bn) { return (int)((long)tn * bn / bm); }
+
+// first row and column of a tile (tile rows vary fastest)
+template <int BM, int BN>
+__device__ __forceinline__ void ztile_origin(const ZGrid& g, bool tri, int tile, int& m0, int& n0) {
+  int tm = tile % g.tiles_m, tn = tile / g.tiles_m;
+  if (tri) {
+    for (tn = 0;; ++tn) {
+      const int first = zfirst_row(tn, BM, BN), count = g.tiles_m - first;
+      if (tile < count) {
+        tm = first + tile;
+        break;
+      }
+      tile -= count;
+    }
+  }
+  m0 = tm * BM;
+  n0 = tn * BN;
+}
+
 // group range of item `it` (split-K)
-__device__ __forceinline__ void zrange(const ZgemmDesc& d, const ZGrid& g, int it, int& g0, int& g1) {
+__device__ __forceinline__ void zrange(const ZgemmDesc& d, const ZGrid& g, int ntile, int it, int& g0, int& g1) {
   g0 = 0;
   g1 = g.groups;
   if (d.splits > 1) {
-    const int split = (it / (g.tiles_m * g.tiles_n)) % d.splits;
+    const int split = (it / ntile) % d.splits;
     g0 = (int)((long)g.groups * split / d.splits);
     g1 = (int)((long)g.groups * (split + 1) / d.splits);
   }
@@ -142,7 +164,9 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
   double2* const As = zsm + team * S * (ASZ + BSZ);
   double2* const Bs = As + S * ASZ;
   const int lane = threadIdx.x & 31;
-  const int ntile = g.tiles_m * g.tiles_n;
+  const bool tri = d.tri && *d.tri;
+  const int ntile = tri ? g.tri_tiles : g.tiles_m * g.tiles_n;
+  const int items = tri ? g.items / (g.tiles_m * g.tiles_n) * g.tri_tiles : g.items;
   // the second round of items starts on other SMs before any SM's second team gets one
   const int it0 = blockIdx.x + team * gridDim.x, stride = gridDim.x * T::TEAMS;
 
@@ -156,15 +180,17 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
     ZRows<B_K, BN, T::CW> rb;
     int t = 0, st = 0;  // steps issued, stage of the next one
     int sa = 0;         // stage of the next announcement
-    for (int it = it0; it < g.items; it += stride) {
+    for (int it = it0; it < items; it += stride) {
       {
         const int tile = it % ntile, batch = it / ntile / d.splits;
         const int b0 = batch % d.nb0, b1 = (batch / d.nb0) % d.nb1, b2 = batch / d.nb0 / d.nb1;
-        ra.begin(d.A + b0 * d.a_b0 + b1 * d.a_b1 + b2 * d.a_b2, d.a_m, d.a_k, (tile % g.tiles_m) * BM, d.M, cl);
-        rb.begin(d.B + b0 * d.b_b0 + b1 * d.b_b1 + b2 * d.b_b2, d.b_n, d.b_k, (tile / g.tiles_m) * BN, d.N, cl);
+        int m0, n0;
+        ztile_origin<BM, BN>(g, tri, tile, m0, n0);
+        ra.begin(d.A + b0 * d.a_b0 + b1 * d.a_b1 + b2 * d.a_b2, d.a_m, d.a_k, m0, d.M, cl);
+        rb.begin(d.B + b0 * d.b_b0 + b1 * d.b_b1 + b2 * d.b_b2, d.b_n, d.b_k, n0, d.N, cl);
       }
       int g0, g1;
-      zrange(d, g, it, g0, g1);
+      zrange(d, g, ntile, it, g0, g1);
       int left = g1 - g0;
       const int kb = g0 / g.gpb;
       int kin = g0 - kb * g.gpb;
@@ -288,7 +314,10 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
     const int tile = it % ntile, rest = it / ntile;
     const int split = rest % d.splits, batch = rest / d.splits;
     const int b0 = batch % d.nb0, b1 = (batch / d.nb0) % d.nb1, b2 = batch / d.nb0 / d.nb1;
-    const int m0 = (tile % g.tiles_m) * BM + wm * 8 * MT + fr, n0 = (tile / g.tiles_m) * BN + wn * 8 * NT + 2 * fk;
+    int m0, n0;
+    ztile_origin<BM, BN>(g, tri, tile, m0, n0);
+    m0 += wm * 8 * MT + fr;
+    n0 += wn * 8 * NT + 2 * fk;
     const bool use_beta = d.beta.x != 0.0 || d.beta.y != 0.0;
     const bool scaled = d.alpha.x != 1.0 || d.alpha.y != 0.0;
     double2* const cb = d.C + b0 * d.c_b0 + b1 * d.c_b1 + b2 * d.c_b2;
@@ -326,12 +355,12 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
   // as soon as its last fragments are in registers
   constexpr int D = T::DB - 1;  // fragment buffer of the second group
   int st = 0;
-  if (it0 < g.items) zbar_sync(FULL, NTHR);
+  if (it0 < items) zbar_sync(FULL, NTHR);
   if (D) load(0, 0, 0);
-  for (int it = it0; it < g.items; it += stride) {
+  for (int it = it0; it < items; it += stride) {
     int g0, g1;
-    zrange(d, g, it, g0, g1);
-    const bool more = it + stride < g.items;
+    zrange(d, g, ntile, it, g0, g1);
+    const bool more = it + stride < items;
     for (int n = g1 - g0; n > 0; n -= 2) {
       if (!D) {
         load(0, st, 0);
