@@ -135,7 +135,11 @@ struct gg_context {
   std::vector<const void*> graph_sig;
   gg::DevBuf<int> gw_flag;  // nonzero: this build's G is Hermitian
   gg::DevBuf<int> gw_err;  // [0] failed, [1] system index (q position x nw_b + Omega), [2] info
-  int plan_qc = 0, plan_kc = 0, plan_tb = 0;  // plan of the eager build, reused by the capture
+  int gw_err_host[3] = {0, 0, 0};
+  // plan of the last eager build (plan_key: precision and spin blocks), reused by later ones and by the capture
+  int plan_key = -1, plan_qc = 0, plan_kc = 0, plan_tb = 0;
+  std::vector<const void*> plan_buffers;  // the work buffers at the end of that build's allocations
+  std::vector<cudaEvent_t> events;  // timing marks of a build
 
   void drop_graph() {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
@@ -154,6 +158,7 @@ struct gg_context {
 
   ~gg_context() {
     drop_graph();
+    for (auto ev : events) cudaEventDestroy(ev);
     if (split) gg::split_release(split);
     if (stream) cudaStreamDestroy(stream);
   }

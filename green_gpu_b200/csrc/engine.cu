@@ -29,34 +29,34 @@ namespace {
 
 inline int64_t tri(long k1, long k2) { return k1 >= k2 ? k1 * (k1 + 1) / 2 + k2 : k2 * (k2 + 1) / 2 + k1; }
 
+// phase marks on a stream, with events that the context keeps between calls
 struct EventTimer {
-  std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> marks;
+  std::vector<std::pair<int, int>> marks;  // (phase, index of its first event)
+  gg_context* c;
   cudaStream_t st;
   bool on;
-  explicit EventTimer(cudaStream_t s, bool enabled = true) : st(s), on(enabled) {}
+  int used = 0;
+  EventTimer(gg_context* ctx, cudaStream_t s, bool enabled) : c(ctx), st(s), on(enabled) {}
   int begin(int id) {
     if (!on) return -1;
-    cudaEvent_t a, b;
-    GG_CUDA(cudaEventCreate(&a));
-    GG_CUDA(cudaEventCreate(&b));
-    GG_CUDA(cudaEventRecord(a, st));
-    marks.push_back({id, {a, b}});
+    while ((int)c->events.size() < used + 2) {
+      cudaEvent_t ev;
+      GG_CUDA(cudaEventCreate(&ev));
+      c->events.push_back(ev);
+    }
+    GG_CUDA(cudaEventRecord(c->events[used], st));
+    marks.push_back({id, used});
+    used += 2;
     return (int)marks.size() - 1;
   }
   void end(int h) {
-    if (h >= 0) GG_CUDA(cudaEventRecord(marks[h].second.second, st));
+    if (h >= 0) GG_CUDA(cudaEventRecord(c->events[marks[h].second + 1], st));
   }
   void collect(double* acc) {
     for (auto& m : marks) {
       float ms = 0;
-      GG_CUDA(cudaEventElapsedTime(&ms, m.second.first, m.second.second));
+      GG_CUDA(cudaEventElapsedTime(&ms, c->events[m.second], c->events[m.second + 1]));
       acc[m.first] += ms * 1e-3;
-    }
-  }
-  ~EventTimer() {
-    for (auto& m : marks) {
-      cudaEventDestroy(m.second.first);
-      cudaEventDestroy(m.second.second);
     }
   }
 };
@@ -234,6 +234,16 @@ Plan plan_gw(gg_context* c, int slices) {
   return p;
 }
 
+namespace {
+
+// the work space that plan_gw() sizes
+std::vector<const void*> work_buffers(const gg_context* c) {
+  return {c->Gf.p,    c->Gtmp.p, c->Vbuf.p, c->G1buf.p, c->scratchA.p, c->scratchB.p, c->P0buf.p,
+          c->Pw.p,    c->Afac.p, c->Wt.p,   c->Wrot.p,  c->gemm_work.p};
+}
+
+}  // namespace
+
 // system index = position of q in this shard's list x nw_b + Omega
 void dyson_failure(const gg_context* c, int solver, int system, int info) {
   const auto& s = c->sh;
@@ -348,10 +358,21 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
     pl.tb = c->plan_tb;
     pl.dyson_batch = 4 * 148;
   } else {
-    pl = plan_gw(c, precision == GG_PREC_SPLIT ? c->slices : 0);
-    c->plan_qc = pl.qc;
-    c->plan_kc = pl.kc;
-    c->plan_tb = pl.tb;
+    // the plan of the previous build of this kind stands while its buffers do: asking for the free
+    // memory again is a driver call that other processes' calls hold up, by tens of milliseconds on a
+    // busy node (a 12.6 ms build took 12.6 to 86 ms)
+    const int key = (precision == GG_PREC_SPLIT ? c->slices : 0) * 8 + ns;
+    if (c->plan_key != key || c->plan_buffers != work_buffers(c)) {
+      c->plan_key = -1;
+      const Plan fresh = plan_gw(c, precision == GG_PREC_SPLIT ? c->slices : 0);
+      c->plan_qc = fresh.qc;
+      c->plan_kc = fresh.kc;
+      c->plan_tb = fresh.tb;
+    }
+    pl.qc = c->plan_qc;
+    pl.kc = c->plan_kc;
+    pl.tb = c->plan_tb;
+    pl.dyson_batch = 4 * 148;
   }
   if (cap && c->profiling) throw Error(GG_ERR_STATE, "gw: profiling is not available while capturing");
   if (cap && (c->cap_P0 || c->cap_Pw || c->cap_Wt)) throw Error(GG_ERR_STATE, "gw: capture of intermediates needs an eager build");
@@ -376,7 +397,10 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
   int* piv = solver == GG_SOLVER_LU ? c->piv.ensure((size_t)dys * N) : nullptr;
   const int lub = dyson_lu_block(N);
   double2* lu_inv = solver == GG_SOLVER_LU ? c->lu_inv.ensure((size_t)dys * ceil_div(N, lub) * lub * lub) : nullptr;
-  std::vector<int> info_h((size_t)pl.qc * nw);
+  if (!cap) {
+    c->plan_key = (precision == GG_PREC_SPLIT ? c->slices : 0) * 8 + ns;
+    c->plan_buffers = work_buffers(c);
+  }
   SplitGemm* split = nullptr;
   if (precision == GG_PREC_SPLIT) split = split_engine(c);
 
@@ -479,9 +503,9 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
   const PairTable& sg_pairs = tables.sg_pairs;
   const IntTable& g1_idx = tables.g1_idx;
   int* gw_err = c->gw_err.ensure(4);
-  if (cap) GG_CUDA(cudaMemsetAsync(gw_err, 0, 4 * sizeof(int), st));
+  GG_CUDA(cudaMemsetAsync(gw_err, 0, 4 * sizeof(int), st));
 
-  EventTimer tm(st, !cap);
+  EventTimer tm(c, st, !cap);
   int h_total = tm.begin(0);
   GG_CUDA(cudaMemsetAsync(Sigma_dev, 0, sizeof(double2) * (size_t)T * ns * s.ink * nn, st));
 
@@ -616,16 +640,10 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
       c->launches += launch_dyson(Pw + (long)s0 * NN, Af, lu_inv, info + s0, sn, N, solver, piv, st);
     }
     tm.end(h);
-    if (cap) {
-      // no host round trip inside a graph: the first failing system is recorded on the device
-      // and reported after the replay (dyson_failure)
-      launch_info_collect(info, qn * nw, q0 * nw, gw_err, st);
-    } else {
-      GG_CUDA(cudaMemcpyAsync(info_h.data(), info, sizeof(int) * qn * nw, cudaMemcpyDeviceToHost, st));
-      GG_CUDA(cudaStreamSynchronize(st));
-      for (int i = 0; i < qn * nw; ++i)
-        if (info_h[i] != 0) dyson_failure(c, solver, q0 * nw + i, info_h[i]);
-    }
+    // no host round trip in the middle of a build: the first failing system is recorded on the device
+    // and reported at the end
+    launch_info_collect(info, qn * nw, q0 * nw, gw_err, st);
+    ++c->launches;
     // ---------------- IR back: Wt[q][t] = sum_w Ttn[t][w] W[q][w]
     h = tm.begin(5);
     {
@@ -745,8 +763,10 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
   }
   tm.end(h_total);
   if (cap) return;  // the caller checks gw_err and the split engine's flag after the replay
-  GG_CUDA(cudaStreamSynchronize(st));
+  GG_CUDA(cudaMemcpyAsync(c->gw_err_host, gw_err, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
   if (split) split_check(split, st);
+  GG_CUDA(cudaStreamSynchronize(st));
+  if (c->gw_err_host[0]) dyson_failure(c, solver, c->gw_err_host[1], c->gw_err_host[2]);
   for (auto& e : kev) {
     float ms = 0;
     GG_CUDA(cudaEventElapsedTime(&ms, e.second.first, e.second.second));

@@ -312,17 +312,23 @@ void launch_x2c_merge(const double2* in, long nouter, long ninner, int n, int nb
 }
 
 namespace {
-__global__ void info_collect_kernel(const int* info, int count, int base, int* err) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-    if (info[i] != 0 && atomicCAS(&err[0], 0, 1) == 0) {
-      err[1] = base + i;
-      err[2] = info[i];
-    }
+__global__ void __launch_bounds__(TPB) info_collect_kernel(const int* info, int count, int base, int* err) {
+  __shared__ int first;
+  if (threadIdx.x == 0) first = count;
+  __syncthreads();
+  for (int i = threadIdx.x; i < count; i += TPB)
+    if (info[i] != 0) atomicMin(&first, i);
+  __syncthreads();
+  if (threadIdx.x == 0 && first < count && err[0] == 0) {
+    err[0] = 1;
+    err[1] = base + first;
+    err[2] = info[first];
+  }
 }
 }  // namespace
 
 void launch_info_collect(const int* info, int count, int base, int* err, cudaStream_t st) {
-  info_collect_kernel<<<grid_for(count), TPB, 0, st>>>(info, count, base, err);
+  info_collect_kernel<<<1, TPB, 0, st>>>(info, count, base, err);
   GG_CHECK_LAUNCH();
 }
 

@@ -21,7 +21,7 @@ void launch_conj_where(double2* X, const int* tr_d, int nk, long per_k, cudaStre
 // gather blocks: out[p][e] = src[idx[p] * src_stride + e] for e < elems
 void launch_gather_blocks(const double2* src, const int* idx_d, int nblocks, long elems, long src_stride,
                           double2* out, cudaStream_t st);
-// err[0..2] <- (1, base + i, info[i]) for a failing system i (info != 0), if none is recorded yet
+// err[0..2] <- (1, base + i, info[i]) for the first failing system i (info != 0), if none is recorded yet
 void launch_info_collect(const int* info, int count, int base, int* err, cudaStream_t st);
 
 // Two-component (X2C) spin blocks.  A spinor matrix of order 2n holds the blocks aa (0,0),
