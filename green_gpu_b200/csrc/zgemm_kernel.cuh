@@ -389,6 +389,7 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
 // kernels hold three accumulators per element, so their tiles are smaller.
 struct ZShape {
   int bm, bn, mt, nt, warps, teams;  // teams resident per SM
+  constexpr bool square() const { return mt == 1 && warps == nt; }
 };
 constexpr ZShape kZShape[] = {
     {64, 64, 4, 4, 4, 2}, {64, 80, 4, 5, 4, 2}, {64, 56, 2, 7, 4, 2}, {64, 48, 2, 6, 4, 2}, {64, 40, 2, 5, 4, 2},
