@@ -61,14 +61,14 @@ struct ZChoice {
   int shape = 0, splits = 1;
 };
 
-// The choice minimises a cycle estimate fitted to timings of every shape and split on 25 of the
+// The choice minimises a cycle estimate fitted to timings of every shape and split on 33 of the
 // library's products (outputs of 20..400 columns, reductions of 20..280000, batches of 1..72; the chosen
-// one is within 2 % of the best measured one on average, 16 % at worst):
+// one is within 2 % of the best measured one on average, 20 % at worst):
 //   pipe   the SM with the most tiles issues tiles x warps/4 x groups x MT NT P DMMAs (P = 4 or 3
 //          products) of 16 cycles on each sub-partition.  The pipe is busy 0.89 - 0.5 / (MT NT) of the
 //          time (V^T W of NQ 400, nao 52, 72 tau: 7.54 ms on 64 x 80 tiles, 8.93 ms on 64 x 16), a fifth
-//          less with three products, which add FP64 sums, and 15 % less on squares of one
-//          warp per row of 8 x 8 tiles; a tile's output costs 150 cycles per 8 x 8 tile;
+//          less with three products, which add FP64 sums, and 10 % less on squares of one
+//          warp per row of 8 x 8 tiles; a tile's output costs 100 cycles per 8 x 8 tile;
 //   chain  groups of one tile follow one another: its DMMAs, or the copy warp's work, per group, and
 //          about 6000 cycles from the first copy to the last store (a 52^3 product: 7.2 us on 16 tiles
 //          of 16 x 16, 17.3 us on one of 64 x 64);
@@ -90,14 +90,14 @@ ZChoice choose(const ZgemmDesc& d, long batch, long groups, int sms) {
     const double tiles = (double)(d.tri ? tri_tiles(tm, tn, s.bm, s.bn) : tm * tn) * batch;
     const int t88 = s.mt * s.nt;
     const double mma = t88 * prods * 16.0, busy =
-        (0.89 - 0.5 / t88) * (d.gauss ? 0.8 : 1.0) * (s.square() ? 0.85 : 1.0);
+        (0.89 - 0.5 / t88) * (d.gauss ? 0.8 : 1.0) * (s.square() ? 0.9 : 1.0);
     const double group = std::max(1.15 * mma + 100.0, 150.0 + 7.0 * (s.bm + s.bn));
     for (int sp : kSplits) {
       if (sp > 1 && (d.inplace || !d.work || groups / sp < 8 || out * sp > (double)d.work_elems)) break;
       const double g = (double)((groups + sp - 1) / sp), items = tiles * sp;
       const double per_sm = std::ceil(items / sms), waves = std::ceil(items / ((double)sms * s.teams));
-      const double pipe = per_sm * s.warps / 4.0 * (g * mma / busy + 150.0 * t88);
-      const double chain = waves * (g * group + 150.0 * t88 + 6000.0);
+      const double pipe = per_sm * s.warps / 4.0 * (g * mma / busy + 100.0 * t88);
+      const double chain = waves * (g * group + 100.0 * t88 + 6000.0);
       const double l2 = per_sm * (s.bm + s.bn) * g * 64.0 / 40.0;
       double cost = std::max(std::max(pipe, chain), l2);
       if (sp > 1) cost += 7000.0 + 100.0 * std::min(sp, 64) + out * (sp + 1) * 16.0 / 3000.0;
@@ -158,6 +158,11 @@ int zgemm(const ZgemmDesc& d0, cudaStream_t stream) {
   g.wrap_a = d.a_kb - 4L * (g.gpb - 1) * d.a_k;
   g.wrap_b = d.b_kb - 4L * (g.gpb - 1) * d.b_k;
   const long teams = std::min<long>(items, (long)sms * s.teams);
+  // start the teams of a paired CTA a tile's DMMA time apart where they walk several short tiles (B-build of P0,
+  // nao 52, NQ 400: 0.96 -> 0.86 ms on 64 x 56 tiles, X G 1.56 -> 1.47 ms on 64 x 64; long tiles hide the output
+  // anyway, and CTAs of one team drift apart by themselves)
+  const double tile_ns = (double)groups / d.splits * s.mt * s.nt * (d.gauss ? 3 : 4) * 16.0 * s.warps / 4 / 1.9;
+  g.stagger = items >= 4 * teams && tile_ns < 200e3 ? (int)tile_ns : 0;
   if (ak && bk) zgemm_launch_kk(ch.shape, d.gauss != 0, d, g, teams, stream);
   else if (ak) zgemm_launch_kn(ch.shape, d.gauss != 0, d, g, teams, stream);
   else if (bk) zgemm_launch_nk(ch.shape, d, g, teams, stream);

@@ -20,7 +20,9 @@
 
 namespace gg {
 
-// Tile shape of one kernel; DB = 2 keeps the next group's fragments in registers.  PAIR: one CTA per SM
+// Tile shape of one kernel.  DB = 2 loads the next group's fragments before the current group's DMMAs issue,
+// which pays only for tiles of one or two DMMA tiles per warp (6 to 20 % there; 4 to 8 % lost on larger
+// ones, whose two warps per sub-partition cover the loads).  PAIR: one CTA per SM
 // holds two independent teams (four DMMA warps, two copy warps and a ring each), and the copy
 // warps hand registers to the DMMA warps (56 and 224 per thread of the 168 that the 384
 // threads are launched with; two CTAs of five warps get 168).
@@ -42,6 +44,7 @@ struct ZGrid {
   int tiles_m, tiles_n;
   int items;            // tiles_m * tiles_n * splits * batch
   int tri_tiles;        // tiles on and below the diagonal
+  int stagger;          // nanoseconds by which the second team of a CTA starts later
   int gpb;              // groups of 4 per K-batch
   int groups;           // KB * gpb
   long wrap_a, wrap_b;  // from the last group of a K-batch to the first of the next
@@ -76,7 +79,7 @@ __host__ __device__ __forceinline__ int zfirst_row(int tn, int bm, int bn) { ret
 // first row and column of a tile (tile rows vary fastest)
 template <int BM, int BN>
 __device__ __forceinline__ void ztile_origin(const ZGrid& g, bool tri, int tile, int& m0, int& n0) {
-  int tm = tile % g.tiles_m, tn = tile / g.tiles_m;
+  int tn = (int)((unsigned)tile / (unsigned)g.tiles_m), tm = tile - tn * g.tiles_m;
   if (tri) {
     for (tn = 0;; ++tn) {
       const int first = zfirst_row(tn, BM, BN), count = g.tiles_m - first;
@@ -89,6 +92,31 @@ __device__ __forceinline__ void ztile_origin(const ZGrid& g, bool tri, int tile,
   }
   m0 = tm * BM;
   n0 = tn * BN;
+}
+
+// tile, split and batch indices of item `it`
+struct ZItem {
+  int tile, split, batch, b0, b1, b2;
+};
+__device__ __forceinline__ ZItem zitem(const ZgemmDesc& d, int ntile, int it) {
+  ZItem w;
+  unsigned rest = (unsigned)it / (unsigned)ntile;
+  w.tile = it - (int)rest * ntile;
+  w.split = 0;
+  if (d.splits > 1) {
+    w.split = (int)(rest % (unsigned)d.splits);
+    rest /= (unsigned)d.splits;
+  }
+  w.batch = (int)rest;
+  w.b0 = w.batch;
+  w.b1 = w.b2 = 0;
+  if (d.nb1 > 1 || d.nb2 > 1) {
+    w.b0 = (int)(rest % (unsigned)d.nb0);
+    rest /= (unsigned)d.nb0;
+    w.b1 = (int)(rest % (unsigned)d.nb1);
+    w.b2 = (int)(rest / (unsigned)d.nb1);
+  }
+  return w;
 }
 
 // group range of item `it` (split-K)
@@ -172,6 +200,8 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
 
   if (copier) {
     if (T::PAIR) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    // teams that start together also write their tiles at the same time, with the DMMA pipe idle
+    if (T::PAIR && team && g.stagger) __nanosleep(g.stagger);
     const int cl = lane + 32 * (T::PAIR ? wid % T::CW : 0);  // lane of the team's copy warps
     // ---------------- copy warp.  Stage t is announced once it has landed and stage t + S - 2 has been
     // issued: the copies of S - 2 stages are in flight, and one landed stage waits for its turn
@@ -182,12 +212,11 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
     int sa = 0;         // stage of the next announcement
     for (int it = it0; it < items; it += stride) {
       {
-        const int tile = it % ntile, batch = it / ntile / d.splits;
-        const int b0 = batch % d.nb0, b1 = (batch / d.nb0) % d.nb1, b2 = batch / d.nb0 / d.nb1;
+        const ZItem w = zitem(d, ntile, it);
         int m0, n0;
-        ztile_origin<BM, BN>(g, tri, tile, m0, n0);
-        ra.begin(d.A + b0 * d.a_b0 + b1 * d.a_b1 + b2 * d.a_b2, d.a_m, d.a_k, m0, d.M, cl);
-        rb.begin(d.B + b0 * d.b_b0 + b1 * d.b_b1 + b2 * d.b_b2, d.b_n, d.b_k, n0, d.N, cl);
+        ztile_origin<BM, BN>(g, tri, w.tile, m0, n0);
+        ra.begin(d.A + w.b0 * d.a_b0 + w.b1 * d.a_b1 + w.b2 * d.a_b2, d.a_m, d.a_k, m0, d.M, cl);
+        rb.begin(d.B + w.b0 * d.b_b0 + w.b1 * d.b_b1 + w.b2 * d.b_b2, d.b_n, d.b_k, n0, d.N, cl);
       }
       int g0, g1;
       zrange(d, g, ntile, it, g0, g1);
@@ -310,45 +339,75 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
         for (int j = 0; j < NT; ++j) dmma(c1[i][j][0], c1[i][j][1], ai[i], fb[buf][j].x);
     }
   };
+  // Output of a tile.  No DMMA issues from this warp meanwhile, so the addresses are kept to one
+  // pointer per row and one column offset that steps by 8 (a division per tile, not per element), and the
+  // usual case - no scaling, no accumulation - has a loop of its own.
   auto epilogue = [&](int it) {
-    const int tile = it % ntile, rest = it / ntile;
-    const int split = rest % d.splits, batch = rest / d.splits;
-    const int b0 = batch % d.nb0, b1 = (batch / d.nb0) % d.nb1, b2 = batch / d.nb0 / d.nb1;
+    const ZItem w = zitem(d, ntile, it);
     int m0, n0;
-    ztile_origin<BM, BN>(g, tri, tile, m0, n0);
+    ztile_origin<BM, BN>(g, tri, w.tile, m0, n0);
     m0 += wm * 8 * MT + fr;
     n0 += wn * 8 * NT + 2 * fk;
+    const bool part = d.splits > 1;
+    const bool plain = part || (d.alpha.x == 1.0 && d.alpha.y == 0.0 && d.beta.x == 0.0 && d.beta.y == 0.0);
     const bool use_beta = d.beta.x != 0.0 || d.beta.y != 0.0;
-    const bool scaled = d.alpha.x != 1.0 || d.alpha.y != 0.0;
-    double2* const cb = d.C + b0 * d.c_b0 + b1 * d.c_b1 + b2 * d.c_b2;
-    double2* const wb = d.work + ((long)split * (d.nb0 * d.nb1 * d.nb2) + batch) * d.M * d.N;
+    double2* const cb = part ? d.work + ((long)w.split * (d.nb0 * d.nb1 * d.nb2) + w.batch) * d.M * d.N
+                             : d.C + w.b0 * d.c_b0 + w.b1 * d.c_b1 + w.b2 * d.c_b2;
     double2* row[MT];
+    bool rok[MT];
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
-      row[i] = d.splits > 1 ? wb + (long)(m0 + i * 8) * d.N : cb + (m0 + i * 8 < d.M ? zmap(d.c_m, m0 + i * 8) : 0);
+    for (int i = 0; i < MT; ++i) {
+      rok[i] = m0 + i * 8 < d.M;
+      row[i] = cb + (!rok[i] ? 0 : part ? (long)(m0 + i * 8) * d.N : zmap(d.c_m, m0 + i * 8));
+    }
+    const int split = part ? 0 : d.c_n.split;
+    const long lo = part ? 1 : d.c_n.lo;
+    const long wrap = split > 0 ? d.c_n.hi - split * lo : 0;
+    auto value = [&](int i, int j, int e) {
+      if constexpr (G3)
+        return make_double2(c0[i][j][e] - c1[i][j][e], c2[i][j][e] - c0[i][j][e] - c1[i][j][e]);
+      else
+        return make_double2(c0[i][j][e], c1[i][j][e]);
+    };
+    int r[2];
+    long off[2];
 #pragma unroll
-    for (int j = 0; j < NT; ++j)
+    for (int e = 0; e < 2; ++e) {
+      r[e] = n0 + e;
+      off[e] = (long)r[e] * lo;
+      if (split > 0) {
+        const int q = r[e] / split;
+        r[e] -= q * split;
+        off[e] = q * d.c_n.hi + r[e] * lo;
+      }
+    }
+    // the two columns of a fragment are written one after the other: they share 32-byte sectors
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (rok[i] && n0 + e + j * 8 < d.N) {
+            double2 v = value(i, j, e);
+            if (!plain) {
+              v = cmul(d.alpha, v);
+              if (use_beta) v = cadd(v, cmul(d.beta, row[i][off[e]]));
+            }
+            row[i][off[e]] = v;
+          }
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int n = n0 + j * 8 + e;
-        if (n >= d.N) continue;
-        const long cn = d.splits > 1 ? n : zmap(d.c_n, n);
-#pragma unroll
-        for (int i = 0; i < MT; ++i) {
-          if (m0 + i * 8 >= d.M) continue;
-          double2 v;
-          if constexpr (G3)
-            v = make_double2(c0[i][j][e] - c1[i][j][e], c2[i][j][e] - c0[i][j][e] - c1[i][j][e]);
-          else
-            v = make_double2(c0[i][j][e], c1[i][j][e]);
-          double2* c = row[i] + cn;
-          if (d.splits == 1) {
-            if (scaled) v = cmul(d.alpha, v);
-            if (use_beta) v = cadd(v, cmul(d.beta, *c));
+        off[e] += 8 * lo;
+        if (split > 0) {
+          r[e] += 8;
+          while (r[e] >= split) {
+            r[e] -= split;
+            off[e] += wrap;
           }
-          *c = v;
         }
       }
+    }
   };
 
   // the barrier in the middle of a step makes the next stage visible; the current one is released
@@ -404,29 +463,29 @@ constexpr int kZShapes = sizeof(kZShape) / sizeof(ZShape), kZShapes3 = sizeof(kZ
 
 template <int I, bool G3>
 struct ZTileOf;
-template <> struct ZTileOf<0, false> { using T = ZTile<4, 4, 2, 2, 1, 3, 2, true>; };
+template <> struct ZTileOf<0, false> { using T = ZTile<4, 4, 2, 2, 1, 3, 1, true>; };
 template <> struct ZTileOf<1, false> { using T = ZTile<4, 5, 2, 2, 1, 3, 1, true>; };
-template <> struct ZTileOf<2, false> { using T = ZTile<2, 7, 4, 1, 1, 3, 2, true>; };
-template <> struct ZTileOf<3, false> { using T = ZTile<2, 6, 4, 1, 1, 3, 2, true>; };
+template <> struct ZTileOf<2, false> { using T = ZTile<2, 7, 4, 1, 1, 3, 1, true>; };
+template <> struct ZTileOf<3, false> { using T = ZTile<2, 6, 4, 1, 1, 3, 1, true>; };
 template <> struct ZTileOf<4, false> { using T = ZTile<2, 5, 4, 1, 2, 4, 1>; };
-template <> struct ZTileOf<5, false> { using T = ZTile<2, 4, 4, 1, 2, 4, 2>; };
-template <> struct ZTileOf<6, false> { using T = ZTile<2, 3, 4, 1, 3, 4, 2>; };
-template <> struct ZTileOf<7, false> { using T = ZTile<2, 2, 4, 1, 4, 4, 2>; };
+template <> struct ZTileOf<5, false> { using T = ZTile<2, 4, 4, 1, 2, 4, 1>; };
+template <> struct ZTileOf<6, false> { using T = ZTile<2, 3, 4, 1, 3, 4, 1>; };
+template <> struct ZTileOf<7, false> { using T = ZTile<2, 2, 4, 1, 4, 4, 1>; };
 template <> struct ZTileOf<8, false> { using T = ZTile<2, 1, 4, 1, 4, 5, 2>; };
 template <> struct ZTileOf<9, false> { using T = ZTile<1, 7, 4, 1, 3, 4, 1>; };
 template <> struct ZTileOf<10, false> { using T = ZTile<1, 7, 7, 1, 2, 7, 1>; };
 template <> struct ZTileOf<11, false> { using T = ZTile<1, 6, 6, 1, 2, 7, 1>; };
 template <> struct ZTileOf<12, false> { using T = ZTile<1, 5, 5, 1, 3, 6, 1>; };
 template <> struct ZTileOf<13, false> { using T = ZTile<1, 3, 3, 1, 4, 7, 2>; };
-template <> struct ZTileOf<14, false> { using T = ZTile<2, 2, 2, 2, 3, 5, 2>; };
+template <> struct ZTileOf<14, false> { using T = ZTile<2, 2, 2, 2, 3, 5, 1>; };
 template <> struct ZTileOf<15, false> { using T = ZTile<1, 1, 2, 2, 4, 7, 2>; };
 template <> struct ZTileOf<0, true> { using T = ZTile<4, 3, 2, 2, 1, 3, 1, true>; };
 template <> struct ZTileOf<1, true> { using T = ZTile<2, 7, 4, 1, 1, 3, 1, true>; };
 template <> struct ZTileOf<2, true> { using T = ZTile<2, 6, 4, 1, 1, 3, 1, true>; };
 template <> struct ZTileOf<3, true> { using T = ZTile<2, 5, 4, 1, 1, 3, 1, true>; };
-template <> struct ZTileOf<4, true> { using T = ZTile<2, 4, 4, 1, 1, 3, 2, true>; };
-template <> struct ZTileOf<5, true> { using T = ZTile<2, 3, 4, 1, 2, 4, 2>; };
-template <> struct ZTileOf<6, true> { using T = ZTile<2, 2, 4, 1, 3, 4, 2>; };
+template <> struct ZTileOf<4, true> { using T = ZTile<2, 4, 4, 1, 1, 3, 1, true>; };
+template <> struct ZTileOf<5, true> { using T = ZTile<2, 3, 4, 1, 2, 4, 1>; };
+template <> struct ZTileOf<6, true> { using T = ZTile<2, 2, 4, 1, 3, 4, 1>; };
 template <> struct ZTileOf<7, true> { using T = ZTile<2, 1, 4, 1, 4, 5, 2>; };
 template <> struct ZTileOf<8, true> { using T = ZTile<1, 7, 4, 1, 3, 4, 1>; };
 template <> struct ZTileOf<9, true> { using T = ZTile<2, 2, 2, 2, 3, 5, 1>; };
