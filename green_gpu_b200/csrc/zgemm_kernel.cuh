@@ -496,6 +496,8 @@ void zgemm_launch_kk(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, lon
 void zgemm_launch_kn(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st);
 void zgemm_launch_nk(int shape, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st);
 void zgemm_launch_nn(int shape, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st);
+// products that do not fill the GPU, any layout: one CTA per 8 x 8 tile (zgemm_small.cu)
+void zgemm_launch_small(const ZgemmDesc& d, const ZGrid& g, cudaStream_t st);
 
 template <class T, bool A_K, bool B_K, bool G3>
 void zlaunch(const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st) {

@@ -22,6 +22,7 @@ def ctx():
 
 @pytest.mark.parametrize("M,N,K", [
     (1, 1, 1), (7, 9, 3), (8, 8, 4), (16, 17, 5), (33, 31, 8), (52, 52, 52), (65, 56, 12),   # one or few tiles
+    (192, 195, 8), (192, 200, 384), (190, 198, 387), (9, 1, 383),                              # small kernel and its limits
     (2000, 7, 9), (1999, 20, 20), (3000, 26, 26), (2050, 37, 41), (4000, 45, 13), (5000, 52, 52),  # one column tile
     (640, 400, 33), (700, 161, 100), (513, 321, 7), (2704, 400, 30),                          # wide tiles
     (64, 64, 4099), (52, 30, 9001), (403, 611, 2707), (9, 700, 1201),                          # split reductions
