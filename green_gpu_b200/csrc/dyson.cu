@@ -8,6 +8,7 @@
 // systems of N = 400 took 31.4 ms and 138 LU systems of N = 251 17.7 ms: too few warps in flight, a
 // barrier every few hundred FMAs, and in the LU one dependent global load per step.
 #include <algorithm>
+#include <type_traits>
 
 #include "dmma.cuh"
 #include "kernels.cuh"
@@ -116,134 +117,184 @@ __global__ void __launch_bounds__(TPB) chol_block_kernel(double2* Aall, int* inf
   if (threadIdx.x == 0 && fail && info[blockIdx.x] == 0) info[blockIdx.x] = fail;
 }
 
-// LU panel: columns j0 .. j0 + nb - 1, rows j0 .. N - 1 of one system, with partial pivoting (largest |re| + |im|,
-// the lowest row on ties), element (row r, column c) of the panel at pan[c * cs + r * rs]: in shared
-// memory by columns when it fits, else in place.  Leaves L below the diagonal block, the
+// LU panel: columns j0 .. j0 + nb - 1 (nb <= 32), rows j0 .. N - 1 of one system, with partial pivoting (largest
+// |re| + |im|, the lowest row on ties), element (row r, column c) of the panel at pan[c * cs + r * rs]: in
+// shared memory by columns when it fits, else in place.  Leaves L below the diagonal block, the
 // block's U^{-1} in its place (zeros below), L^{-1} of the block in li (unit diagonal, zeros above),
 // and the row interchanges (absolute rows) in piv.
-__global__ void __launch_bounds__(TPB) lu_panel_kernel(double2* Aall, double2* li_all, long li_sys, int* piv_all, int* info,
+// Bound by the chain of columns (FP64 latencies, not throughput).  Warp k % 8 owns column k, lanes go down the
+// rows; the owner of column c + 1 updates it first, finds its pivot within the warp and scales it while
+// the other warps still apply column c, so that a column costs one barrier.  With all threads on rows, a
+// block-wide FP64 search and two barriers per column a panel of 69 systems of N = 140 took 67 us, now 54;
+// of 552 systems of N = 120 159 and 129 us.
+__device__ __forceinline__ double2 cinv(double2 d) {
+  const double dn = d.x * d.x + d.y * d.y;
+  if (!(dn > 0.0)) return make_double2(0.0, 0.0);
+  const double f = 1.0 / dn;
+  return make_double2(d.x * f, -d.y * f);
+}
+
+__global__ void __launch_bounds__(TPB, 2) lu_panel_kernel(double2* Aall, double2* li_all, long li_sys, int* piv_all, int* info,
                                                        int N, int j0, int nb, int in_smem) {
   extern __shared__ __align__(16) double2 dsm[];
-  __shared__ double red_v[TPB / 32];
-  __shared__ int red_i[TPB / 32];
-  const int tid = threadIdx.x, lane = tid & 31;
+  __shared__ int s_piv[32];
+  __shared__ int s_fail;
+  constexpr int W = TPB / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double2* A = Aall + blockIdx.x * (long)N * N + (long)j0 * N + j0;
-  int* piv = piv_all + (long)blockIdx.x * N + j0;
   const int R = N - j0;
   const long cs = in_smem ? (R | 1) : 1, rs = in_smem ? 1 : N;
   double2* pan = in_smem ? dsm : A;
-  if (in_smem) {
-    for (int e = tid; e < R * nb; e += TPB) pan[(e % nb) * cs + e / nb] = A[(long)(e / nb) * N + e % nb];
-    __syncthreads();
-  }
-  double best = -1.0;
-  int bi = 0;
-  for (int r = tid; r < R; r += TPB) {
-    const double2 x = pan[r * rs];
-    const double m = fabs(x.x) + fabs(x.y);
-    if (m > best) {
-      best = m;
-      bi = r;
-    }
-  }
-  int fail = 0;
-  for (int c = 0; c < nb; ++c) {
-    // largest entry of column c at or below the diagonal
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) {
-        best = ov;
-        bi = oi;
+  if (tid == 0) s_fail = 0;
+  if (in_smem && lane < nb)
+    for (int r = warp; r < R; r += W) pan[lane * cs + r] = A[(long)r * N + lane];
+  __syncthreads();
+  // pivot of column c (owner warp only): search rows >= c, interchange inside the column, scale
+  auto pivot = [&](int c) {
+    double2* col = pan + c * cs;
+    // magnitudes compared as the bits of non-negative doubles: three warp reductions (high word, low
+    // word, lowest row) instead of five rounds of FP64 comparisons; a NaN counts as zero
+    unsigned hi = 0, lo = 0;
+    int bi = c;
+    for (int r = lane; r < R; r += 32) {
+      const double2 x = col[r * rs];
+      const double m = fabs(x.x) + fabs(x.y);
+      const unsigned long long bits = r >= c && m == m ? __double_as_longlong(m) : 0;
+      const unsigned h = (unsigned)(bits >> 32), w = (unsigned)bits;
+      if (h > hi || (h == hi && w > lo)) {
+        hi = h;
+        lo = w;
+        bi = r;
       }
     }
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    const bool some = mh != 0 || ml != 0;
+    const int p = some ? (int)__reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? (unsigned)bi : 0xffffffffu) : c;
+    const double2 d = col[p * rs];
+    const double2 top = col[c * rs];
+    __syncwarp();
     if (lane == 0) {
-      red_v[tid >> 5] = best;
-      red_i[tid >> 5] = bi;
+      col[p * rs] = top;
+      col[c * rs] = d;
+      s_piv[c] = p;
+      if (!some && s_fail == 0) s_fail = j0 + c + 1;
     }
-    __syncthreads();
-    best = red_v[0];
-    bi = red_i[0];
-    for (int w = 1; w < TPB / 32; ++w)
-      if (red_v[w] > best || (red_v[w] == best && red_i[w] < bi)) {
-        best = red_v[w];
-        bi = red_i[w];
+    __syncwarp();
+    const double2 inv = cinv(d);
+    for (int r0 = lane; r0 < R; r0 += 128) {
+      double2 x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = r0 + 32 * i < R ? col[(r0 + 32 * i) * rs] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = cmul(x[i], inv);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (r0 + 32 * i > c && r0 + 32 * i < R) col[(r0 + 32 * i) * rs] = x[i];
+    }
+  };
+  // column c applied to Q of this warp's columns, k0, k0 + W, ...: all loads of a step before its stores,
+  // so that the FP64 latencies overlap
+  auto update = [&](int c, int k0, auto count) {
+    constexpr int Q = decltype(count)::value;
+    const double2* l = pan + c * cs;
+    double2 u[Q];
+    double2* col[Q];
+    bool ok[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      ok[q] = k0 + W * q < nb;
+      col[q] = pan + (ok[q] ? k0 + W * q : c) * cs;
+      u[q] = col[q][c * rs];
+    }
+    for (int r0 = lane; r0 < R; r0 += 64) {
+      double2 lv[2], x[2][Q];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int r = r0 + 32 * i < R ? r0 + 32 * i : R - 1;
+        lv[i] = l[r * rs];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) x[i][q] = col[q][r * rs];
       }
-    const int p = best < 0.0 ? c : bi;  // no comparable entry (NaN): keep the row
-    if (!(best > 0.0) && !fail) fail = j0 + c + 1;
-    if (tid == 0) piv[c] = j0 + p;
-    if (tid < nb && p != c) {
-      const double2 x = pan[tid * cs + c * rs];
-      pan[tid * cs + c * rs] = pan[tid * cs + p * rs];
-      pan[tid * cs + p * rs] = x;
-    }
-    __syncthreads();
-    const double2 d = pan[c * cs + c * rs];
-    const double dn = d.x * d.x + d.y * d.y;
-    const double2 inv = dn > 0.0 ? make_double2(d.x / dn, -d.y / dn) : make_double2(0.0, 0.0);
-    best = -1.0;
-    bi = c + 1;
-    for (int r = tid; r < R; r += TPB) {
-      if (r <= c) continue;
-      const double2 l = cmul(pan[c * cs + r * rs], inv);
-      pan[c * cs + r * rs] = l;
-      for (int k = c + 1; k < nb; ++k) {
-        const double2 x = csub(pan[k * cs + r * rs], cmul(l, pan[k * cs + c * rs]));
-        pan[k * cs + r * rs] = x;
-        if (k == c + 1) {
-          const double m = fabs(x.x) + fabs(x.y);
-          if (m > best) {
-            best = m;
-            bi = r;
-          }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int r = r0 + 32 * i;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          x[i][q] = csub(x[i][q], cmul(lv[i], u[q]));
+          if (ok[q] && r > c && r < R) col[q][r * rs] = x[i][q];
         }
       }
     }
-  }
+  };
+  if (warp == 0) pivot(0);
   __syncthreads();
-  if (in_smem)
-    for (int e = tid; e < R * nb; e += TPB)
-      if (e / nb >= nb) A[(long)(e / nb) * N + e % nb] = pan[(e % nb) * cs + e / nb];
-  // the block's inverses: T = the block, X = L^{-1}, Y = U^{-1}, built by row operations on the identity
+  for (int c = 0; c < nb; ++c) {
+    const int p = s_piv[c];
+    const int k = warp + W * lane;  // the warp's columns: one lane interchanges each
+    if (k < nb && k != c && p != c) {
+      const double2 x = pan[k * cs + c * rs];
+      pan[k * cs + c * rs] = pan[k * cs + p * rs];
+      pan[k * cs + p * rs] = x;
+    }
+    __syncwarp();
+    const bool next = c + 1 < nb && (c + 1) % W == warp;
+    if (next) {
+      update(c, c + 1, std::integral_constant<int, 1>());
+      __syncwarp();
+      pivot(c + 1);
+    }
+    // the warp's columns beyond c (and beyond c + 1 where that one is done), from the first such k
+    const int first = c + (next ? 2 : 1);
+    const int k0 = first + (warp - first % W + W) % W, left = (nb - k0 + W - 1) / W;
+    if (left > 2) update(c, k0, std::integral_constant<int, 4>());
+    else if (left == 2) update(c, k0, std::integral_constant<int, 2>());
+    else if (left == 1) update(c, k0, std::integral_constant<int, 1>());
+    __syncthreads();
+  }
+  int* piv = piv_all + (long)blockIdx.x * N + j0;
+  if (tid < nb) piv[tid] = j0 + s_piv[tid];
+  if (in_smem && lane < nb)
+    for (int r = nb + warp; r < R; r += W) A[(long)r * N + lane] = pan[lane * cs + r];
+  // the block's inverses X = L^{-1} and Y = U^{-1}, built by row operations on the identity: T holds L below the
+  // diagonal and U D^{-1} above it (D the diagonal of U), Y's rows are scaled at the end
   double2 t[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int e = tid + i * TPB, r = e / 32, c = e % 32;
+    const int r = warp + W * i, c = lane;
     t[i] = r < nb && c < nb ? pan[c * cs + r * rs] : make_double2(r == c ? 1.0 : 0.0, 0.0);
+    if (r < c && c < nb) t[i] = cmul(t[i], cinv(pan[c * cs + c * rs]));
   }
   __syncthreads();
   double2 (*T)[33] = reinterpret_cast<double2 (*)[33]>(dsm);
   double2 (*X)[33] = T + 32, (*Y)[33] = T + 64;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int e = tid + i * TPB, r = e / 32, c = e % 32;
+    const int r = warp + W * i, c = lane;
     T[r][c] = t[i];
-    X[r][c] = make_double2(r == c ? 1.0 : 0.0, 0.0);
-    Y[r][c] = make_double2(r == c ? 1.0 : 0.0, 0.0);
+    X[r][c] = Y[r][c] = make_double2(r == c ? 1.0 : 0.0, 0.0);
   }
   __syncthreads();
   for (int c = 0; c < nb; ++c) {
     const int b = nb - 1 - c;  // pivot row of the upper solve
-    const double2 d = T[b][b];
-    const double dn = d.x * d.x + d.y * d.y;
-    const double2 inv = dn > 0.0 ? make_double2(d.x / dn, -d.y / dn) : make_double2(0.0, 0.0);
-    if (tid < 32) Y[b][tid] = cmul(Y[b][tid], inv);
-    __syncthreads();
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int e = tid + i * TPB, r = e / 32, k = e % 32;
+      const int r = warp + W * i, k = lane;
       if (r > c && k <= c) X[r][k] = csub(X[r][k], cmul(T[r][c], X[c][k]));
       if (r < b && k >= b) Y[r][k] = csub(Y[r][k], cmul(T[r][b], Y[b][k]));
     }
     __syncthreads();
   }
   double2* li = li_all + blockIdx.x * li_sys;
-  for (int e = tid; e < nb * nb; e += TPB) {
-    const int r = e / nb, c = e % nb;
-    li[e] = X[r][c];
-    A[(long)r * N + c] = Y[r][c];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = warp + W * i, c = lane;
+    if (r < nb && c < nb) {
+      li[r * nb + c] = X[r][c];
+      A[(long)r * N + c] = cmul(cinv(T[r][r]), Y[r][c]);
+    }
   }
-  if (tid == 0 && fail && info[blockIdx.x] == 0) info[blockIdx.x] = fail;
+  if (tid == 0 && s_fail && info[blockIdx.x] == 0) info[blockIdx.x] = s_fail;
 }
 
 // Row interchanges of a panel on the columns outside it (y = 0: A) and on the right-hand side (y = 1: P):
