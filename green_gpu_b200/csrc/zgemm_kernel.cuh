@@ -381,21 +381,33 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
         off[e] = q * d.c_n.hi + r[e] * lo;
       }
     }
-    // the two columns of a fragment are written one after the other: they share 32-byte sectors
+    // a lane's two columns are neighbours in memory where C is contiguous along n: one 32-byte store (a full
+    // sector) where the address allows it, else one after the other, since they share sectors
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
+      const bool ok0 = n0 + j * 8 < d.N, ok1 = n0 + j * 8 + 1 < d.N;
 #pragma unroll
-      for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-          if (rok[i] && n0 + e + j * 8 < d.N) {
-            double2 v = value(i, j, e);
-            if (!plain) {
-              v = cmul(d.alpha, v);
-              if (use_beta) v = cadd(v, cmul(d.beta, row[i][off[e]]));
-            }
-            row[i][off[e]] = v;
+      for (int i = 0; i < MT; ++i) {
+        if (!rok[i]) continue;
+        double2* const p0 = row[i] + off[0];
+        double2* const p1 = row[i] + off[1];
+        double2 v0 = value(i, j, 0), v1 = value(i, j, 1);
+        if (!plain) {
+          v0 = cmul(d.alpha, v0);
+          v1 = cmul(d.alpha, v1);
+          if (use_beta) {
+            if (ok0) v0 = cadd(v0, cmul(d.beta, *p0));
+            if (ok1) v1 = cadd(v1, cmul(d.beta, *p1));
           }
+        }
+        if (ok1 && p1 == p0 + 1 && ((size_t)p0 & 31) == 0) {
+          asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p0), "d"(v0.x), "d"(v0.y), "d"(v1.x), "d"(v1.y)
+                       : "memory");
+        } else {
+          if (ok0) *p0 = v0;
+          if (ok1) *p1 = v1;
+        }
+      }
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         off[e] += 8 * lo;
