@@ -989,33 +989,65 @@ std::vector<int> widths(int S) {
   return {64};
 }
 
+// split-K factor that fills whole waves of persistent CTAs with `base` units of nkb K blocks (each split keeps
+// >= 8): fewer splits unless a larger count fills the machine noticeably better
+int wave_splits(long base, int nkb) {
+  const int smax = (int)std::max<long>(1, std::min<long>(nkb / 8, 64));
+  int splits = 1;
+  double best = 0.0;
+  for (int sp = 1; sp <= smax; ++sp) {
+    const long units = base * sp;
+    const long waves = (units + sms() - 1) / sms();
+    const double eff = (double)units / (double)(waves * sms());
+    if (eff > best + 0.05) {
+      best = eff;
+      splits = sp;
+    }
+    if (units >= 4L * sms()) break;
+  }
+  return splits;
+}
+
+// Tile width (B' rows per tile; it changes no element's arithmetic).  Accumulators of S diagonals x BN columns must
+// fit the 512 TMEM columns, and BN <= 128 keeps the FP64 drain registers (BN / 2 per thread) in budget.
+// Where several fit, the one with the least waves x (BN + 30): a tile's time grows with its width beyond a fixed
+// part worth about 30 columns (the reads of A and the ends of the pipeline).  Against the least padding
+// alone: NQ 251 P0 199 -> 148 us (64 -> 96 wide, one wave without split-K), operand builds of nao 37
+// 0.20 -> 0.15 ms (48 -> 96), Sigma of NQ 400 stays at 80.  A single K block (nao <= 32 operand builds) is all drain,
+// where 96 columns per tile cost more than they save: nao 26 99 -> 88 us with 80.
+int tile_width(const ZgemmDesc& d, int S, const Geometry& g) {
+  if (S <= 4) return 128;
+  if (S > 6) return 64;
+  const int cands[4] = {80, 96, 64, 48};
+  const long tiles_m = (d.M + BM - 1) / BM;
+  double best = -1.0;
+  int width = 80;
+  for (int bn : cands) {
+    if (S == 6 && (bn == 96 || bn == 48)) continue;
+    if (S == 5 && g.nkb == 1 && bn < 80) continue;
+    const long base = tiles_m * ((2L * d.N + bn - 1) / bn) * g.batch;
+    const int sp = wave_splits(base, g.nkb);
+    const double waves = (double)((base * sp + sms() - 1) / sms()) / sp;
+    const double cost = waves * (bn + (g.nkb == 1 ? 0 : 30));
+    if (best < 0.0 || cost < best) {
+      best = cost;
+      width = bn;
+    }
+  }
+  return width;
+}
+
 Geometry geometry(const ZgemmDesc& d, int S, int force_bn = 0) {
   if (S < 2 || S > 8) throw Error(GG_ERR_ARG, "split: slices must be in [2, 8]");
   Geometry g;
-  // nbuf accumulator sets of S diagonals x BN columns must fit the 512 TMEM columns;
-  // BN <= 128 keeps the FP64 drain registers (BN / 2 per thread) in budget
-  // tile width: the widest one whose accumulators fit TMEM, or a narrower one that pads the
-  // 2N rows of B' less (2N = 800: 80 divides it, 96 pads it to 864)
-  g.BN = S <= 4 ? 128 : S == 5 ? 96 : S == 6 ? 80 : 64;
-  if (S == 5 || S == 6) {
-    const int cands[4] = {96, 80, 64, 48};
-    long best = -1;
-    for (int bn : cands) {
-      if (S == 6 && (bn == 96 || bn == 48)) continue;
-      const long pad = ((2L * d.N + bn - 1) / bn) * bn;
-      if (best < 0 || pad < best) {
-        best = pad;
-        g.BN = bn;
-      }
-    }
-  }
   g.batch = (long)d.nb0 * d.nb1 * d.nb2;
   g.Ktot = (long)d.KB * d.K;
   if (2 * g.Ktot + KB >= (1L << 31) || (long)d.M >= (1L << 31) || (long)d.N >= (1L << 30))
     throw Error(GG_ERR_ARG, "split: operand dimensions too large for one launch");
   g.kp = ((2 * g.Ktot + KB - 1) / KB) * KB;
   g.rows_a_pad = ((d.M + BM - 1) / BM) * BM;
-  if (force_bn) g.BN = force_bn;
+  g.nkb = (int)(g.kp / KB);
+  g.BN = force_bn ? force_bn : tile_width(d, S, g);
   // two accumulator sets when they fit TMEM: the next tile's MMAs then run while the epilogue
   // drains the previous tile (S <= 2, or 48-wide tiles at 5 slices)
   g.nbuf = 2 * S * g.BN <= 512 ? 2 : 1;
@@ -1025,7 +1057,6 @@ Geometry geometry(const ZgemmDesc& d, int S, int force_bn = 0) {
   // exact int32 chunk: S * Kchunk * 64^2 < 2^31 (slices are rounded, |d| <= 64)
   const long kchunk = std::max<long>(KB, ((2147483647L / (4096L * S)) / KB) * KB);
   g.kcb = (int)(kchunk / KB);
-  g.nkb = (int)(g.kp / KB);
   return g;
 }
 
@@ -1086,25 +1117,12 @@ int run_planes(SplitGemm* e, const ZgemmDesc& d, int S, const Geometry& g, const
   if (a.stages < 2) throw Error(GG_ERR_ARG, "split: stage does not fit shared memory");
   const size_t smem = a.stages * stage_bytes + 1024 + 512;  // + alignment + barriers and TMEM slot
   const long base = (long)a.tiles_m * a.tiles_n * g.batch;
-  // split-K so that the units fill whole waves of persistent CTAs (each split keeps >= 8 K
-  // blocks); the row-max epilogue needs whole reductions (no split-K)
+  // the row-max epilogue needs whole reductions (no split-K)
   int splits = 1;
   if (force_splits > 0) {
     splits = a.mx.on ? 1 : force_splits;
   } else if (!a.mx.on) {
-    const int smax = (int)std::max<long>(1, std::min<long>(g.nkb / 8, 64));
-    double best = 0.0;
-    for (int sp = 1; sp <= smax; ++sp) {
-      const long units = base * sp;
-      const long waves = (units + sms() - 1) / sms();
-      const double eff = (double)units / (double)(waves * sms());
-      // prefer fewer splits unless a larger count fills the machine noticeably better
-      if (eff > best + 0.05) {
-        best = eff;
-        splits = sp;
-      }
-      if (units >= 4L * sms()) break;
-    }
+    splits = wave_splits(base, g.nkb);
   }
   const long need = (long)d.M * d.N * g.batch;
   if (splits > 1) {
@@ -1238,20 +1256,7 @@ int sliced_gemm(SplitGemm* e, const ZgemmDesc& d, int S, cudaStream_t st, const 
     gc.rows_b_plane = g.rows_b_plane;
     gc.ncol_pad = g.ncol_pad;
     const long base = (long)(gc.rows_a_pad / BM) * (gc.rows_b_pad / bn) * gc.batch;
-    int rule = 1;
-    {
-      const int smax = (int)std::max<long>(1, std::min<long>(gc.nkb / 8, 64));
-      double b = 0.0;
-      for (int sp = 1; sp <= smax; ++sp) {
-        const long units = base * sp, waves = (units + sms() - 1) / sms();
-        const double eff = (double)units / (double)(waves * sms());
-        if (eff > b + 0.05) {
-          b = eff;
-          rule = sp;
-        }
-        if (units >= 4L * sms()) break;
-      }
-    }
+    const int rule = wave_splits(base, gc.nkb);
     const int smax = mx ? 1 : (int)std::max<long>(1, std::min<long>(gc.nkb / 8, 64));
     std::vector<int> sps{rule, 1, std::min(2 * rule, smax)};
     std::sort(sps.begin(), sps.end());
