@@ -195,7 +195,7 @@ Plan plan_gw(gg_context* c, int slices) {
     b += 2 * std::max(p0s, sgs);
     b += (size_t)q.qc * T2 * NN;                       // P0
     b += (size_t)q.qc * s.nw_b * NN;                   // Pw
-    b += (size_t)std::min<long>(q.dyson_batch, (long)q.qc * s.nw_b) * (NN + 32 * (size_t)s.NQ);  // Dyson workspace
+    b += (size_t)std::min<long>(q.dyson_batch, (long)q.qc * s.nw_b) * NN;  // Dyson workspace
     b += (size_t)q.qc * s.nts * NN;                    // Wt
     b += (size_t)s.nts * NN;                           // Wrot
     b += (size_t)1 << 22;                              // split-K partials
@@ -832,7 +832,10 @@ void hf_exchange(gg_context* c, const double2* dm_dev, double2* K_dev, cudaStrea
   c->Gtmp.ensure((size_t)nk * ns * nn);
   // pairs per step: all k2 of as many irreducible k as 256 MB of integrals hold (at least one, so that
   // a small system takes few launches), or k2 in chunks when the device has less room than that
-  const int krc = (int)std::max<long>(1, std::min<long>(s.ink, (256L << 20) / ((long)nk * Nnn * (long)sizeof(double2))));
+  // the split engine's slice planes (rows of n padded to a 128-row tile) count towards the same 256 MB
+  const long per_k = (long)nk * Nnn * (long)sizeof(double2) +
+                     (c->hf_precision == GG_PREC_SPLIT ? 2L * c->slices * nk * N * n * (128 + 2 * n) : 0);
+  const int krc = (int)std::max<long>(1, std::min<long>(s.ink, (256L << 20) / per_k));
   int kc = nk, kg = krc;  // k2 and irreducible k per step
   const size_t want = (size_t)krc * nk * Nnn;
   if (c->Vbuf.n < want || c->scratchA.n < want) {
