@@ -73,6 +73,11 @@ __device__ __forceinline__ void zbar_arrive(int id, int threads) {
   asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// two neighbouring elements as one 32-byte store
+__device__ __forceinline__ void zstore2(double2* p, double2 v0, double2 v1) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v0.x), "d"(v0.y), "d"(v1.x), "d"(v1.y) : "memory");
+}
+
 // tile row that holds the diagonal of tile column tn: the first one of a lower-triangle product
 __host__ __device__ __forceinline__ int zfirst_row(int tn, int bm, int bn) { return (int)((long)tn * bn / bm); }
 
@@ -360,15 +365,39 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
       rok[i] = m0 + i * 8 < d.M;
       row[i] = cb + (!rok[i] ? 0 : part ? (long)(m0 + i * 8) * d.N : zmap(d.c_m, m0 + i * 8));
     }
-    const int split = part ? 0 : d.c_n.split;
-    const long lo = part ? 1 : d.c_n.lo;
-    const long wrap = split > 0 ? d.c_n.hi - split * lo : 0;
     auto value = [&](int i, int j, int e) {
       if constexpr (G3)
         return make_double2(c0[i][j][e] - c1[i][j][e], c2[i][j][e] - c0[i][j][e] - c1[i][j][e]);
       else
         return make_double2(c0[i][j][e], c1[i][j][e]);
     };
+    const int split = part ? 0 : d.c_n.split;
+    const long lo = part ? 1 : d.c_n.lo;
+    // short reductions into contiguous rows (X G): a row's pointer and immediate offsets.  They spend a third of a
+    // tile's instructions on its output (X G of nao 52 1.24 -> 1.22 ms, with three products 1.07 -> 1.03, nao 37
+    // 0.31 -> 0.29, nao 20 49.9 -> 45.9 us); the other layouts have long reductions, where the second loop
+    // only costs registers (Z V^+ of nao 52 0.84 -> 0.90 ms)
+    if (A_K && !B_K && plain && split == 0 && lo == 1) {
+      const int left = d.N - n0;
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        if (!rok[i]) continue;
+        double2* const p = row[i] + n0;
+        const bool wide = ((size_t)p & 31) == 0;  // columns step by 8: the same for the whole row
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          const double2 v0 = value(i, j, 0), v1 = value(i, j, 1);
+          if (wide && j * 8 + 1 < left) {
+            zstore2(p + j * 8, v0, v1);
+          } else {
+            if (j * 8 < left) p[j * 8] = v0;
+            if (j * 8 + 1 < left) p[j * 8 + 1] = v1;
+          }
+        }
+      }
+      return;
+    }
+    const long wrap = split > 0 ? d.c_n.hi - split * lo : 0;
     int r[2];
     long off[2];
 #pragma unroll
@@ -401,8 +430,7 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
           }
         }
         if (ok1 && p1 == p0 + 1 && ((size_t)p0 & 31) == 0) {
-          asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p0), "d"(v0.x), "d"(v0.y), "d"(v1.x), "d"(v1.y)
-                       : "memory");
+          zstore2(p0, v0, v1);
         } else {
           if (ok0) *p0 = v0;
           if (ok1) *p1 = v1;
