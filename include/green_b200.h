@@ -130,8 +130,9 @@ int gg_set_split_slices(gg_context* ctx, int slices);
  * registers, for nao <= 52 (larger orbital counts use the two GEMMs); enable = 0 (default) runs
  * the two GEMMs, with Z in device memory, as src/cugw_qkpt.cu:295-332 does.  The fused form
  * saves Z's write and read (2 x nts x NQ x nao^2 x 16 bytes per (k, q) pair), but both forms
- * are bound by the DMMA issue rate, and at nao 52, NQ 400 the fused kernel takes 2.64 ms per
- * pair against 2.54 ms for the two GEMMs.  Both sum in a fixed order (deterministic); they
+ * are bound by the FP64 tensor pipe, which the fused kernel keeps 59 % busy and the GEMMs 80 to
+ * 92 %: at nao 52, NQ 400 it takes 2.64 ms per pair against 1.87 ms for the two GEMMs (2.96
+ * against 2.26 ms in FP64 builds).  Both sum in a fixed order (deterministic); they
  * differ in the FP64 summation order only. */
 int gg_set_fused_tail(gg_context* ctx, int enable);
 
