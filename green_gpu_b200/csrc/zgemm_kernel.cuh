@@ -485,19 +485,21 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) zgemm_kernel(const __grid
 // 64 x 8 NT and 32 x 8 NT serve outputs of at most 56 columns (N = nao), where one tile spans the
 // width; squares of 24, 32, 40, 48 and 56 serve nao x nao outputs of long reductions (exchange), 16 x 16
 // products whose few tiles would leave most SMs idle.  The three-product
-// kernels hold three accumulators per element, so their tiles are smaller.
+// kernels hold three accumulators per element, so their tiles are smaller.  Each shape has as many
+// CTAs per SM as its registers allow (64 x 32: two -> three, operand build of nao 26 95 -> 87 us, Z V^+ of nao 20
+// 64 -> 50 us; a fourth CTA of 64 x 24 lost 3 % on V^T W and exchange products).
 struct ZShape {
   int bm, bn, mt, nt, warps, teams;  // teams resident per SM
   constexpr bool square() const { return mt == 1 && warps == nt; }
 };
 constexpr ZShape kZShape[] = {
     {64, 64, 4, 4, 4, 2}, {64, 80, 4, 5, 4, 2}, {64, 56, 2, 7, 4, 2}, {64, 48, 2, 6, 4, 2}, {64, 40, 2, 5, 4, 2},
-    {64, 32, 2, 4, 4, 2}, {64, 24, 2, 3, 4, 3}, {64, 16, 2, 2, 4, 4}, {64, 8, 2, 1, 4, 4}, {32, 56, 1, 7, 4, 3},
+    {64, 32, 2, 4, 4, 3}, {64, 24, 2, 3, 4, 3}, {64, 16, 2, 2, 4, 4}, {64, 8, 2, 1, 4, 4}, {32, 56, 1, 7, 4, 3},
     {56, 56, 1, 7, 7, 2}, {48, 48, 1, 6, 6, 2}, {40, 40, 1, 5, 5, 3}, {24, 24, 1, 3, 3, 4}, {32, 32, 2, 2, 4, 3},
     {16, 16, 1, 1, 4, 4}};
 constexpr ZShape kZShape3[] = {
     {64, 48, 4, 3, 4, 2}, {64, 56, 2, 7, 4, 2}, {64, 48, 2, 6, 4, 2}, {64, 40, 2, 5, 4, 2}, {64, 32, 2, 4, 4, 2},
-    {64, 24, 2, 3, 4, 2}, {64, 16, 2, 2, 4, 3}, {64, 8, 2, 1, 4, 4}, {32, 56, 1, 7, 4, 3}, {32, 32, 2, 2, 4, 3},
+    {64, 24, 2, 3, 4, 3}, {64, 16, 2, 2, 4, 3}, {64, 8, 2, 1, 4, 4}, {32, 56, 1, 7, 4, 3}, {32, 32, 2, 2, 4, 3},
     {16, 16, 1, 1, 4, 4}};
 constexpr int kZShapes = sizeof(kZShape) / sizeof(ZShape), kZShapes3 = sizeof(kZShape3) / sizeof(ZShape);
 
@@ -508,7 +510,7 @@ template <> struct ZTileOf<1, false> { using T = ZTile<4, 5, 2, 2, 1, 3, 1, true
 template <> struct ZTileOf<2, false> { using T = ZTile<2, 7, 4, 1, 1, 3, 1, true>; };
 template <> struct ZTileOf<3, false> { using T = ZTile<2, 6, 4, 1, 1, 3, 1, true>; };
 template <> struct ZTileOf<4, false> { using T = ZTile<2, 5, 4, 1, 2, 4, 1>; };
-template <> struct ZTileOf<5, false> { using T = ZTile<2, 4, 4, 1, 2, 4, 1>; };
+template <> struct ZTileOf<5, false> { using T = ZTile<2, 4, 4, 1, 3, 4, 1>; };
 template <> struct ZTileOf<6, false> { using T = ZTile<2, 3, 4, 1, 3, 4, 1>; };
 template <> struct ZTileOf<7, false> { using T = ZTile<2, 2, 4, 1, 4, 4, 1>; };
 template <> struct ZTileOf<8, false> { using T = ZTile<2, 1, 4, 1, 4, 5, 2>; };
@@ -524,7 +526,7 @@ template <> struct ZTileOf<1, true> { using T = ZTile<2, 7, 4, 1, 1, 3, 1, true>
 template <> struct ZTileOf<2, true> { using T = ZTile<2, 6, 4, 1, 1, 3, 1, true>; };
 template <> struct ZTileOf<3, true> { using T = ZTile<2, 5, 4, 1, 1, 3, 1, true>; };
 template <> struct ZTileOf<4, true> { using T = ZTile<2, 4, 4, 1, 1, 3, 1, true>; };
-template <> struct ZTileOf<5, true> { using T = ZTile<2, 3, 4, 1, 2, 4, 1>; };
+template <> struct ZTileOf<5, true> { using T = ZTile<2, 3, 4, 1, 3, 4, 1>; };
 template <> struct ZTileOf<6, true> { using T = ZTile<2, 2, 4, 1, 3, 4, 1>; };
 template <> struct ZTileOf<7, true> { using T = ZTile<2, 1, 4, 1, 4, 5, 2>; };
 template <> struct ZTileOf<8, true> { using T = ZTile<1, 7, 4, 1, 3, 4, 1>; };
