@@ -244,6 +244,26 @@ std::vector<const void*> work_buffers(const gg_context* c) {
 
 }  // namespace
 
+// Number of tau (a divisor of T) whose rows (tau, Q) form one GEMM: the fewest that leave at most 1 % of
+// their tiles of 64 rows empty, else those that leave least, as long as the operands of the group stay in L2
+// (64 MB of W~).  V^T W of 72 tau: NQ 160, nao 20 220 -> 209 us (400 x 160 per tau in tiles of 64 x 80, now 320 x 400
+// of two tau), NQ 182, nao 26 464 -> 429 us, NQ 400, nao 52 7.51 -> 7.40 ms.
+int tau_rows(int T, int N) {
+  int best = 1;
+  double least = 2.0;
+  for (int tb = 1; tb <= T; ++tb) {
+    const long rows = (long)tb * N;
+    if (T % tb || (tb > 1 && rows * N * (long)sizeof(double2) > (64L << 20)) || rows > (1L << 30)) continue;
+    const double waste = (double)((rows + 63) / 64 * 64) / rows - 1.0;
+    if (waste < least - 1e-12) {
+      best = tb;
+      least = waste;
+    }
+    if (least <= 0.01) break;
+  }
+  return best;
+}
+
 // system index = position of q in this shard's list x nw_b + Omega
 void dyson_failure(const gg_context* c, int solver, int system, int info) {
   const auto& s = c->sh;
@@ -667,6 +687,7 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
     const bool fused_tail = c->fused_tail && sigma_tail_supported(n, T, (long)c->gemm_work.n);
     const double tail_flops = (double)T * (8.0 * N * n * (double)nn + 12.0 * N * (double)nn) +
                               8.0 * T * n * (double)n * N * n + 12.0 * T * (double)nn;
+    const int tb = tau_rows(T, N);
     for (int qi = 0; qi < qn; ++qi) {
       const int iq = myq[q0 + qi];
       for (int qd : c->q_stars[iq]) {
@@ -674,17 +695,20 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
         const double2* W = Wt + (long)qi * T * NN;
         if (c->has_Uq) {
           // Wr[t] = U_q' W[t] U_q'^+, once per star member (cugw_qkpt.cu:297-318 does it per (k,t))
+          // (rows (tau, column) resp. (tau, row): the rotation is the shared operand)
           ZgemmDesc d;
-          d.M = N; d.N = N; d.K = N;
-          d.A = c->Uq.p + (long)qd * NN; d.a_m.lo = N; d.a_k = 1;
-          d.B = W; d.b_k = N; d.b_n.lo = 1;
-          d.C = SA; d.c_m.lo = N; d.c_n.lo = 1;
-          d.nb0 = T; d.a_b0 = 0; d.b_b0 = NN; d.c_b0 = NN;
+          d.M = tb * N; d.N = N; d.K = N;
+          d.A = W; d.a_m.split = N; d.a_m.hi = NN; d.a_m.lo = 1; d.a_k = N;
+          d.B = c->Uq.p + (long)qd * NN; d.b_k = 1; d.b_n.lo = N;
+          d.C = SA; d.c_m.split = N; d.c_m.hi = NN; d.c_m.lo = 1; d.c_n.lo = N;
+          d.nb0 = T / tb; d.a_b0 = tb * NN; d.b_b0 = 0; d.c_b0 = tb * NN;
           gemm(d);
-          ZgemmDesc e = d;
-          e.A = SA; e.a_b0 = NN;
-          e.B = c->Uq.p + (long)qd * NN; e.b_k = 1; e.b_n.lo = N; e.conjB = 1; e.b_b0 = 0;
-          e.C = Wr;
+          ZgemmDesc e;
+          e.M = tb * N; e.N = N; e.K = N;
+          e.A = SA; e.a_m.lo = N; e.a_k = 1;
+          e.B = c->Uq.p + (long)qd * NN; e.b_k = 1; e.b_n.lo = N; e.conjB = 1;
+          e.C = Wr; e.c_m.lo = N; e.c_n.lo = 1;
+          e.nb0 = T / tb; e.a_b0 = tb * NN; e.b_b0 = 0; e.c_b0 = tb * NN;
           gemm(e);
           W = Wr;
         }
@@ -697,11 +721,20 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
           // of the tau batch (sliced once in split precision) and X serves every spin.
           {
             ZgemmDesc d;
-            d.M = (int)nn; d.N = N; d.K = N;
-            d.A = Vb; d.a_m.lo = 1; d.a_k = nn;
-            d.B = W; d.b_k = N; d.b_n.lo = 1; d.conjB = trq ? 1 : 0;
-            d.C = SA; d.c_m.lo = 1; d.c_n.lo = nn;
-            d.nb0 = T; d.a_b0 = 0; d.b_b0 = NN; d.c_b0 = Nnn;
+            if (split) {
+              d.M = (int)nn; d.N = N; d.K = N;
+              d.A = Vb; d.a_m.lo = 1; d.a_k = nn;
+              d.B = W; d.b_k = N; d.b_n.lo = 1; d.conjB = trq ? 1 : 0;
+              d.C = SA; d.c_m.lo = 1; d.c_n.lo = nn;
+              d.nb0 = T; d.a_b0 = 0; d.b_b0 = NN; d.c_b0 = Nnn;
+            } else {
+              // transposed: rows (tau, Q) of a few tau fill whole tiles of 64 (tau_rows), columns x
+              d.M = tb * N; d.N = (int)nn; d.K = N;
+              d.A = W; d.a_m.split = N; d.a_m.hi = NN; d.a_m.lo = 1; d.a_k = N; d.conjA = trq ? 1 : 0;
+              d.B = Vb; d.b_k = nn; d.b_n.lo = 1;
+              d.C = SA; d.c_m.lo = nn; d.c_n.lo = 1;
+              d.nb0 = T / tb; d.a_b0 = tb * NN; d.b_b0 = 0; d.c_b0 = tb * Nnn;
+            }
             // W' is the same for every k of this star member: in split precision it is sliced for the
             // first one (the tail below runs on the FP64 engine, so the slices stay in place).  At nao
             // 52, NQ 400 its exponents and slices took 0.07 + 0.10 ms of a pair's 3.9 ms
