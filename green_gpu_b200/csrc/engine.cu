@@ -533,16 +533,26 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
   int h = tm.begin(1);
   // With Hermitian G(tau), as a physical one is, every k's term of P0 is Hermitian whatever V is
   // (conj Tr[G^k V^Q G^k1 V^Q'+] = Tr[G^k V^Q' G^k1 V^Q+]), so its lower triangle is enough.  The device
-  // looks at this call's G; any other G takes all tiles.  FP64 only: the split product's errors above and
-  // below the diagonal are independent, and the Dyson step's averaging of the two halves is
-  // part of its accuracy (Sigma 8.3e-10 instead of 5.9e-10 from the lower triangle alone).
+  // looks at this call's G; any other G takes all tiles.  A G that is Hermitian only to rounding (2^-46)
+  // enters P0 as its Hermitian part Gp: what the Dyson step's averaging of the two halves of the full P0
+  // drops is just the first order of the rest, which the lower triangle alone would keep (1e-14 of
+  // Sigma at the limit; the second order is 2^-92).  A caller that looks at P0 itself, before that
+  // averaging, gets the full one unless G is Hermitian to 8 units in the last place.  FP64 only: the split product's
+  // errors above and below the diagonal are independent, and averaging them is part of its accuracy
+  // (Sigma 8.3e-10 instead of 5.9e-10 from the lower triangle alone).
   int* herm = nullptr;
   if (!split) {
     herm = c->gw_flag.ensure(1);
-    launch_hermitian_check(G_dev, T, ns, s.ink, n, c->x2c, herm, st);
+    launch_hermitian_check(G_dev, T, ns, s.ink, n, c->x2c, c->cap_P0 ? 0x1p-49 : 0x1p-46, herm, st);
     ++c->launches;
   }
   unfold_matrices(c, G_dev, T, ns, Gf, st);
+  const double2* Gp = Gf;
+  if (!split) {
+    Gp = c->Gtmp.p;  // free once G is unfolded
+    launch_hermitian_part(Gf, nk, ns, T, n, c->x2c, herm, c->Gtmp.p, st);
+    ++c->launches;
+  }
   tm.end(h);
 
   const double pref = ns == 1 ? -2.0 : -1.0;
@@ -562,11 +572,11 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
         ++c->launches;
         for (int sp = 0; sp < ns; ++sp) {
           // G1[kk][t] = G^{k+q}(tau_t), t < T/2
-          launch_gather_blocks(Gf, g1_idx.d.p + ((size_t)iq * ns + sp) * nk + k0, kn, (long)T2 * nn, (long)T * nn,
+          launch_gather_blocks(Gp, g1_idx.d.p + ((size_t)iq * ns + sp) * nk + k0, kn, (long)T2 * nn, (long)T * nn,
                                G1, st);
           ++c->launches;
           if (split) {
-            p0_split_block(c, split, Gf, G1, Vb, SA, SB, P0 + (long)qi * T2 * NN, k0, kn, spin_a(sp), pl, pref,
+            p0_split_block(c, split, Gp, G1, Vb, SA, SB, P0 + (long)qi * T2 * NN, k0, kn, spin_a(sp), pl, pref,
                            (sp == 0 && k0 == 0), st, [&](const ZgemmDesc& d, const int* ea, const int* eb) {
                              const Exps pr{ea, eb};
                              gemm_main(d, 0, true, &pr);
@@ -581,7 +591,7 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
             {
               ZgemmDesc d;
               d.M = tn * n; d.N = N * n; d.K = n;
-              d.A = Gf + ((long)k0 * ns + spin_a(sp)) * T * nn + (long)(T - 1 - t0) * nn;
+              d.A = Gp + ((long)k0 * ns + spin_a(sp)) * T * nn + (long)(T - 1 - t0) * nn;
               d.a_m.split = n; d.a_m.hi = -nn; d.a_m.lo = n; d.a_k = 1;
               d.B = Vb; d.b_k = n; d.b_n.split = n; d.b_n.hi = nn; d.b_n.lo = 1;
               d.C = SA; d.c_m.split = n; d.c_m.hi = Nnn; d.c_m.lo = n;

@@ -102,9 +102,9 @@ __global__ void scale_kernel(double2* X, long n, double s) {
 }
 
 // One CTA per matrix (blockIdx.x = (t * ns + s) * ink + k): clears *flag unless G[t][s][k] and G[t][s'][k]^H agree
-// within 2^-46 of the largest element of either, s' = s or, with `swap` (X2C spin blocks), 0, 1, 3, 2
+// within tol of the largest element of either, s' = s or, with `swap` (X2C spin blocks), 0, 1, 3, 2
 __global__ void __launch_bounds__(128) hermitian_check_kernel(const double2* __restrict__ G, int ns, int ink, int n, int swap,
-                                                              int* flag) {
+                                                              double tol, int* flag) {
   __shared__ double red[2][4];
   const long nn = (long)n * n;
   const long b = blockIdx.x;
@@ -136,7 +136,37 @@ __global__ void __launch_bounds__(128) hermitian_check_kernel(const double2* __r
       big = fmax(big, red[0][w]);
       off = fmax(off, red[1][w]);
     }
-    if (any_bad || off > 0x1p-46 * big) *flag = 0;
+    if (any_bad || off > tol * big) *flag = 0;
+  }
+}
+
+// One CTA per 32 x 32 tile of a matrix (blockIdx.x = (k * ns + s) * nts + t): H = (G + G'^H) / 2 where *flag, else G, with
+// G'(s) as in the check.  Reads every tile and its mirror once each, through shared memory (HBM-bound).
+__global__ void __launch_bounds__(TPB) hermitian_part_kernel(const double2* __restrict__ G, int ns, int nts, int n, int swap,
+                                                             const int* flag, double2* __restrict__ H) {
+  __shared__ double2 m[32][33];
+  const int tiles = (n + 31) / 32, ti = blockIdx.y / tiles, tj = blockIdx.y % tiles;
+  const long b = blockIdx.x, nn = (long)n * n;
+  const int s = (int)((b / nts) % ns), p = swap && s >= 2 ? 5 - s : s;
+  const double2* X = G + b * nn;
+  const double2* Y = X + (long)(p - s) * nts * nn;
+  const bool half = *flag != 0;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  if (half)
+    for (int r = ty; r < 32; r += 8) {
+      const int i = tj * 32 + r, j = ti * 32 + tx;
+      if (i < n && j < n) m[r][tx] = Y[(long)i * n + j];
+    }
+  __syncthreads();
+  for (int r = ty; r < 32; r += 8) {
+    const int i = ti * 32 + r, j = tj * 32 + tx;
+    if (i >= n || j >= n) continue;
+    double2 x = X[(long)i * n + j];
+    if (half) {
+      const double2 y = m[tx][r];
+      x = make_double2(0.5 * (x.x + y.x), 0.5 * (x.y - y.y));
+    }
+    H[b * nn + (long)i * n + j] = x;
   }
 }
 
@@ -340,9 +370,17 @@ void launch_transpose_blocks(const double2* in, long nblocks, int n, double2* ou
   GG_CHECK_LAUNCH();
 }
 
-void launch_hermitian_check(const double2* G, int nts, int ns, int ink, int n, int swap, int* flag, cudaStream_t st) {
+void launch_hermitian_check(const double2* G, int nts, int ns, int ink, int n, int swap, double tol, int* flag,
+                            cudaStream_t st) {
   GG_CUDA(cudaMemsetAsync(flag, 1, sizeof(int), st));
-  hermitian_check_kernel<<<nts * ns * ink, 128, 0, st>>>(G, ns, ink, n, swap, flag);
+  hermitian_check_kernel<<<nts * ns * ink, 128, 0, st>>>(G, ns, ink, n, swap, tol, flag);
+  GG_CHECK_LAUNCH();
+}
+
+void launch_hermitian_part(const double2* G, int nk, int ns, int nts, int n, int swap, const int* flag, double2* H,
+                           cudaStream_t st) {
+  const int t = ceil_div(n, 32);
+  hermitian_part_kernel<<<dim3(nk * ns * nts, t * t), TPB, 0, st>>>(G, ns, nts, n, swap, flag, H);
   GG_CHECK_LAUNCH();
 }
 

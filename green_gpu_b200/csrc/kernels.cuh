@@ -38,9 +38,13 @@ void launch_x2c_merge(const double2* in, long nouter, long ninner, int n, int nb
 // out[b][i][j] = in[b][j][i] for nblocks n x n matrices (32 x 32 tiles through shared memory)
 void launch_transpose_blocks(const double2* in, long nblocks, int n, double2* out, cudaStream_t st);
 
-// *flag (device) = nonzero when every G[t][s][k] (layout [nts][ns][ink][n][n]) is Hermitian to rounding, else 0; swap: blocks 2
-// and 3 are each other's adjoints (X2C)
-void launch_hermitian_check(const double2* G, int nts, int ns, int ink, int n, int swap, int* flag, cudaStream_t st);
+// *flag (device) = nonzero when every G[t][s][k] (layout [nts][ns][ink][n][n]) is Hermitian within tol of its largest element,
+// else 0; swap: blocks 2 and 3 are each other's adjoints (X2C)
+void launch_hermitian_check(const double2* G, int nts, int ns, int ink, int n, int swap, double tol, int* flag,
+                            cudaStream_t st);
+// H = the Hermitian parts of G (layout [nk][ns][nts][n][n]) where *flag (device), else a copy
+void launch_hermitian_part(const double2* G, int nk, int ns, int nts, int n, int swap, const int* flag, double2* H,
+                           cudaStream_t st);
 // where *flag (device): the upper triangles of nmat n x n matrices from their lower ones
 void launch_mirror_lower(double2* X, int nmat, int n, const int* flag, cudaStream_t st);
 
