@@ -117,10 +117,10 @@ __global__ void __launch_bounds__(128) hermitian_check_kernel(const double2* __r
     const int i = e / n, j = e - i * n;
     const double2 x = X[e], y = Y[(long)j * n + i];
     const double m = fmax(fmax(fabs(x.x), fabs(x.y)), fmax(fabs(y.x), fabs(y.y)));
-    const double o = fmax(fabs(x.x - y.x), fabs(x.y + y.y));
-    bad = bad || !(o <= 1e300);  // NaN and infinities
+    const double dr = fabs(x.x - y.x), di = fabs(x.y + y.y);
+    bad = bad || !(dr <= 1e300) || !(di <= 1e300);  // NaN and infinities, each by itself: fmax drops a NaN
     big = fmax(big, m);
-    off = fmax(off, o);
+    off = fmax(off, fmax(dr, di));
   }
   for (int o = 16; o > 0; o >>= 1) {
     big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
