@@ -23,18 +23,20 @@ constexpr int LU_SMEM = 220 * 1024;
 
 // Hermitian symmetrisation in place, M = (M + M^H) / 2 with a real diagonal
 // (cuda_common.cu:249-281); with A != NULL also A = I - M (cu_compute_Pq.cu:44-63), its lower
-// triangle only when `lower`.  One 32 x 32 tile pair per CTA: both tiles pass through shared memory,
+// triangle only when `lower`.  One CTA per system (fastest) and pair of 32 x 32 tiles, in one grid dimension since
+// N > 11552 has more pairs than the second one takes: both tiles pass through shared memory,
 // so that every access to global memory is a run of 32 elements.
-__global__ void __launch_bounds__(TPB) hermitize_kernel(double2* Pall, double2* Aall, int* info, int N, int lower) {
+__global__ void __launch_bounds__(TPB) hermitize_kernel(double2* Pall, double2* Aall, int* info, int nsys, int N, int lower) {
   __shared__ double2 lo[32][33], up[32][33];
-  int ti = 0, p = blockIdx.y;
+  const int sys = blockIdx.x % nsys;
+  int ti = 0, p = blockIdx.x / nsys;
+  if (info && p == 0 && threadIdx.x == 0) info[sys] = 0;
   while (p > ti) p -= ++ti;  // pair (ti, p), p <= ti
   const int tj = p;  // tj <= ti
   const long NN = (long)N * N;
-  double2* P = Pall + blockIdx.x * NN;
-  double2* A = Aall ? Aall + blockIdx.x * NN : nullptr;
+  double2* P = Pall + sys * NN;
+  double2* A = Aall ? Aall + sys * NN : nullptr;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  if (info && blockIdx.y == 0 && threadIdx.x == 0) info[blockIdx.x] = 0;
   for (int r = ty; r < 32; r += 8) {
     const int i = ti * 32 + r, j = tj * 32 + tx;
     if (i < N && j < N) lo[r][tx] = P[(long)i * N + j];
@@ -406,7 +408,7 @@ int lu(double2* P, double2* A, double2* li, int* info, int* piv, int nsys, int N
 
 void hermitize(double2* P, double2* A, int* info, int nsys, int N, int lower, cudaStream_t st) {
   const int t = ceil_div(N, 32);
-  hermitize_kernel<<<dim3(nsys, t * (t + 1) / 2), TPB, 0, st>>>(P, A, info, N, lower);
+  hermitize_kernel<<<(unsigned)((long)nsys * t * (t + 1) / 2), TPB, 0, st>>>(P, A, info, nsys, N, lower);
   GG_CHECK_LAUNCH();
 }
 

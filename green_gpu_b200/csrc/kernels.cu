@@ -140,13 +140,13 @@ __global__ void __launch_bounds__(128) hermitian_check_kernel(const double2* __r
   }
 }
 
-// One CTA per 32 x 32 tile of a matrix (blockIdx.x = (k * ns + s) * nts + t): H = (G + G'^H) / 2 where *flag, else G, with
+// One CTA per matrix b = (k * ns + s) * nts + t, b < nmat (fastest), and 32 x 32 tile: H = (G + G'^H) / 2 where *flag, else G, with
 // G'(s) as in the check.  Reads every tile and its mirror once each, through shared memory (HBM-bound).
-__global__ void __launch_bounds__(TPB) hermitian_part_kernel(const double2* __restrict__ G, int ns, int nts, int n, int swap,
-                                                             const int* flag, double2* __restrict__ H) {
+__global__ void __launch_bounds__(TPB) hermitian_part_kernel(const double2* __restrict__ G, int nmat, int ns, int nts, int n,
+                                                             int swap, const int* flag, double2* __restrict__ H) {
   __shared__ double2 m[32][33];
-  const int tiles = (n + 31) / 32, ti = blockIdx.y / tiles, tj = blockIdx.y % tiles;
-  const long b = blockIdx.x, nn = (long)n * n;
+  const int tiles = (n + 31) / 32, tile = blockIdx.x / nmat, ti = tile / tiles, tj = tile % tiles;
+  const long b = blockIdx.x % nmat, nn = (long)n * n;
   const int s = (int)((b / nts) % ns), p = swap && s >= 2 ? 5 - s : s;
   const double2* X = G + b * nn;
   const double2* Y = X + (long)(p - s) * nts * nn;
@@ -170,13 +170,14 @@ __global__ void __launch_bounds__(TPB) hermitian_part_kernel(const double2* __re
   }
 }
 
-// where *flag: X[b][i][j] = conj(X[b][j][i]) above the diagonal and a real diagonal; one 32 x 32 tile pair per CTA
-__global__ void __launch_bounds__(TPB) mirror_lower_kernel(double2* X, int n, const int* flag) {
+// where *flag: X[b][i][j] = conj(X[b][j][i]) above the diagonal and a real diagonal; one CTA per matrix
+// (fastest) and 32 x 32 tile pair
+__global__ void __launch_bounds__(TPB) mirror_lower_kernel(double2* X, int nmat, int n, const int* flag) {
   __shared__ double2 s[32][33];
   if (!*flag) return;
-  int ti = 0, tj = blockIdx.y;
+  int ti = 0, tj = blockIdx.x / nmat;
   while (tj > ti) tj -= ++ti;  // tile row ti >= tile column tj
-  double2* M = X + blockIdx.x * (long)n * n;
+  double2* M = X + blockIdx.x % nmat * (long)n * n;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int r = ty; r < 32; r += 8) {
     const int i = ti * 32 + r, j = tj * 32 + tx;
@@ -380,13 +381,14 @@ void launch_hermitian_check(const double2* G, int nts, int ns, int ink, int n, i
 void launch_hermitian_part(const double2* G, int nk, int ns, int nts, int n, int swap, const int* flag, double2* H,
                            cudaStream_t st) {
   const int t = ceil_div(n, 32);
-  hermitian_part_kernel<<<dim3(nk * ns * nts, t * t), TPB, 0, st>>>(G, ns, nts, n, swap, flag, H);
+  const int nmat = nk * ns * nts;
+  hermitian_part_kernel<<<(unsigned)((long)nmat * t * t), TPB, 0, st>>>(G, nmat, ns, nts, n, swap, flag, H);
   GG_CHECK_LAUNCH();
 }
 
 void launch_mirror_lower(double2* X, int nmat, int n, const int* flag, cudaStream_t st) {
   const int t = ceil_div(n, 32);
-  mirror_lower_kernel<<<dim3(nmat, t * (t + 1) / 2), TPB, 0, st>>>(X, n, flag);
+  mirror_lower_kernel<<<(unsigned)((long)nmat * t * (t + 1) / 2), TPB, 0, st>>>(X, nmat, n, flag);
   GG_CHECK_LAUNCH();
 }
 
