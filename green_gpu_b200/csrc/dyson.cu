@@ -135,6 +135,9 @@ __global__ void __launch_bounds__(TPB) chol_block_kernel(double2* Aall, int* inf
 __device__ __forceinline__ double2 cinv(double2 d) {
   const double dn = d.x * d.x + d.y * d.y;
   if (!(dn > 0.0)) return make_double2(0.0, 0.0);
+  // 1 / dn overflows for |d| below 7e-155, where the inverse itself is still finite: quotients there (everywhere they
+  // would lengthen the chain of columns: gamma-point build of NQ 140 1.36 -> 1.39 ms)
+  if (dn < 0x1p-1000) return make_double2(d.x / dn, -d.y / dn);
   const double f = 1.0 / dn;
   return make_double2(d.x * f, -d.y * f);
 }
