@@ -136,8 +136,9 @@ struct gg_context {
   gg::DevBuf<int> gw_flag;  // nonzero: this build's G is Hermitian
   gg::DevBuf<int> gw_err;  // [0] failed, [1] system index (q position x nw_b + Omega), [2] info
   int gw_err_host[3] = {0, 0, 0};
-  // plan of the last eager build (plan_key: precision and spin blocks), reused by later ones and by the capture
-  int plan_key = -1, plan_qc = 0, plan_kc = 0, plan_tb = 0;
+  // plan of the last eager build (plan_key: precision, spin blocks and solver), reused by later ones and by the capture
+  gg::Plan plan;
+  int plan_key = -1;
   std::vector<const void*> plan_buffers;  // the work buffers at the end of that build's allocations
   std::vector<cudaEvent_t> events;  // timing marks of a build
 

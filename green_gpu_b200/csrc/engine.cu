@@ -174,17 +174,18 @@ void x2c_check(const gg_context* c) {
                             "time-reversal partners)");
 }
 
-Plan plan_gw(gg_context* c, int slices) {
-  const auto& s = c->sh;
-  const int nspin = gw_spins(c);
+Plan plan_work(const gg_shape& s, int nspin, int slices, int solver, size_t budget) {
   const size_t z = sizeof(double2);
   const size_t nn = (size_t)s.nao * s.nao, NN = (size_t)s.NQ * s.NQ, Nnn = (size_t)s.NQ * nn;
   const int T2 = s.nts / 2;
-  const size_t held = c->Gf.n + c->Gtmp.n + c->Vbuf.n + c->G1buf.n + c->scratchA.n + c->scratchB.n + c->P0buf.n +
-                      c->Pw.n + c->Afac.n + c->Wt.n + c->Wrot.n + c->gemm_work.n + c->lu_inv.n;
-  const size_t budget = (size_t)(0.85 * (double)(free_bytes() + held * z));
   Plan p;
-  p.dyson_batch = 4 * 148;
+  p.dyson_batch = (int)std::min<long>(4 * 148, (long)s.inq * s.nw_b);
+  // LU: inverses of the diagonal blocks of a batch of systems
+  auto lu_bytes = [&](const Plan& q) {
+    if (solver != GG_SOLVER_LU) return (size_t)0;
+    const size_t lub = dyson_lu_block(s.NQ);
+    return z * (size_t)std::min<long>(q.dyson_batch, (long)q.qc * s.nw_b) * ceil_div(s.NQ, (long)lub) * lub * lub;
+  };
   auto need = [&](const Plan& q) {
     size_t b = 0;
     b += 2 * (size_t)s.nk * nspin * s.nts * nn;       // Gf + Gtmp
@@ -222,16 +223,24 @@ Plan plan_gw(gg_context* c, int slices) {
       }
     }
   }
-  while (need(p) > budget) {
+  while (need(p) + lu_bytes(p) > budget) {
     if (p.qc > 1) p.qc = (p.qc + 1) / 2;
     else if (p.tb > 1) p.tb = (p.tb + 1) / 2;
     else if (p.kc > 1) p.kc = (p.kc + 1) / 2;
+    else if (std::min(p.dyson_batch, s.nw_b) > 1) p.dyson_batch = (std::min(p.dyson_batch, s.nw_b) + 1) / 2;
+    else if (need(p) <= budget) break;  // one system's inverses: within the part of the memory outside the budget
     else
       throw Error(GG_ERR_MEMORY, "GW build does not fit the device: need " + std::to_string(need(p) >> 20) +
                                      " MiB of work space, budget " + std::to_string(budget >> 20) + " MiB");
   }
-  p.bytes = need(p);
+  p.bytes = need(p) + lu_bytes(p);
   return p;
+}
+
+Plan plan_gw(gg_context* c, int slices, int solver) {
+  const size_t held = c->Gf.n + c->Gtmp.n + c->Vbuf.n + c->G1buf.n + c->scratchA.n + c->scratchB.n + c->P0buf.n +
+                      c->Pw.n + c->Afac.n + c->Wt.n + c->Wrot.n + c->gemm_work.n + c->lu_inv.n;
+  return plan_work(c->sh, gw_spins(c), slices, solver, (size_t)(0.85 * (double)(free_bytes() + held * sizeof(double2))));
 }
 
 namespace {
@@ -239,7 +248,7 @@ namespace {
 // the work space that plan_gw() sizes
 std::vector<const void*> work_buffers(const gg_context* c) {
   return {c->Gf.p,    c->Gtmp.p, c->Vbuf.p, c->G1buf.p, c->scratchA.p, c->scratchB.p, c->P0buf.p,
-          c->Pw.p,    c->Afac.p, c->Wt.p,   c->Wrot.p,  c->gemm_work.p};
+          c->Pw.p,    c->Afac.p, c->Wt.p,   c->Wrot.p,  c->gemm_work.p, c->lu_inv.p};
 }
 
 }  // namespace
@@ -370,30 +379,18 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
   // (copy_Gk_2c with minus_t = true, gw_gpu_kernel.cpp:523-536)
   auto spin_a = [&](int sp) { return (c->x2c && sp >= 2) ? 5 - sp : sp; };
   const bool cap = c->capturing;
-  Plan pl;
-  if (cap) {
-    // the captured build replays the eager build's chunking, so every buffer already exists
-    pl.qc = c->plan_qc;
-    pl.kc = c->plan_kc;
-    pl.tb = c->plan_tb;
-    pl.dyson_batch = 4 * 148;
-  } else {
+  const int plan_key = ((precision == GG_PREC_SPLIT ? c->slices : 0) * 8 + ns) * 2 + (solver == GG_SOLVER_LU);
+  if (!cap) {
     // the plan of the previous build of this kind stands while its buffers do: asking for the free
     // memory again is a driver call that other processes' calls hold up, by tens of milliseconds on a
     // busy node (a 12.6 ms build took 12.6 to 86 ms)
-    const int key = (precision == GG_PREC_SPLIT ? c->slices : 0) * 8 + ns;
-    if (c->plan_key != key || c->plan_buffers != work_buffers(c)) {
+    if (c->plan_key != plan_key || c->plan_buffers != work_buffers(c)) {
       c->plan_key = -1;
-      const Plan fresh = plan_gw(c, precision == GG_PREC_SPLIT ? c->slices : 0);
-      c->plan_qc = fresh.qc;
-      c->plan_kc = fresh.kc;
-      c->plan_tb = fresh.tb;
+      c->plan = plan_gw(c, precision == GG_PREC_SPLIT ? c->slices : 0, solver);
     }
-    pl.qc = c->plan_qc;
-    pl.kc = c->plan_kc;
-    pl.tb = c->plan_tb;
-    pl.dyson_batch = 4 * 148;
   }
+  // the captured build replays the eager build's chunking, so every buffer already exists
+  const Plan pl = c->plan;
   if (cap && c->profiling) throw Error(GG_ERR_STATE, "gw: profiling is not available while capturing");
   if (cap && (c->cap_P0 || c->cap_Pw || c->cap_Wt)) throw Error(GG_ERR_STATE, "gw: capture of intermediates needs an eager build");
   c->launches = 0;
@@ -418,7 +415,7 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
   const int lub = dyson_lu_block(N);
   double2* lu_inv = solver == GG_SOLVER_LU ? c->lu_inv.ensure((size_t)dys * ceil_div(N, lub) * lub * lub) : nullptr;
   if (!cap) {
-    c->plan_key = (precision == GG_PREC_SPLIT ? c->slices : 0) * 8 + ns;
+    c->plan_key = plan_key;
     c->plan_buffers = work_buffers(c);
   }
   SplitGemm* split = nullptr;

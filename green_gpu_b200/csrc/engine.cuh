@@ -5,7 +5,9 @@
 
 namespace gg {
 
-Plan plan_gw(gg_context* c, int slices);
+// chunks of a GW build whose work space takes at most `budget` bytes (slices: 0 in FP64 builds)
+Plan plan_work(const gg_shape& s, int nspin, int slices, int solver, size_t budget);
+Plan plan_gw(gg_context* c, int slices, int solver);
 // spin blocks the GW / HF engines loop over: ns, or the X2C pseudo-spins (4 for GW, 3 for HF)
 int gw_spins(const gg_context* c);
 // irreducible q points of shard `rank` of `size`: iq = rank, rank + size, ... (cugw_utils.cu:115)
