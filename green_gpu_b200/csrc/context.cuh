@@ -46,6 +46,7 @@ struct Plan {
   int tb = 1;   // tau points per P0 batch
   int dyson_batch = 1;  // Dyson systems per launch
   size_t bytes = 0;
+  bool whole = false;  // nothing had to be cut into smaller chunks for lack of memory
 };
 
 struct Timings {

@@ -223,6 +223,7 @@ Plan plan_work(const gg_shape& s, int nspin, int slices, int solver, size_t budg
       }
     }
   }
+  p.whole = need(p) + lu_bytes(p) <= budget;
   while (need(p) + lu_bytes(p) > budget) {
     if (p.qc > 1) p.qc = (p.qc + 1) / 2;
     else if (p.tb > 1) p.tb = (p.tb + 1) / 2;
@@ -383,8 +384,9 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
   if (!cap) {
     // the plan of the previous build of this kind stands while its buffers do: asking for the free
     // memory again is a driver call that other processes' calls hold up, by tens of milliseconds on a
-    // busy node (a 12.6 ms build took 12.6 to 86 ms)
-    if (c->plan_key != plan_key || c->plan_buffers != work_buffers(c)) {
+    // busy node (a 12.6 ms build took 12.6 to 86 ms).  A plan that memory cut short is made anew each time, since
+    // the memory may be free by then
+    if (!c->plan.whole || c->plan_key != plan_key || c->plan_buffers != work_buffers(c)) {
       c->plan_key = -1;
       c->plan = plan_gw(c, precision == GG_PREC_SPLIT ? c->slices : 0, solver);
     }
