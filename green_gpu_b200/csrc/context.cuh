@@ -136,7 +136,13 @@ struct gg_context {
   std::vector<const void*> graph_sig;
   gg::DevBuf<int> gw_flag;  // nonzero: this build's G is Hermitian
   gg::DevBuf<int> gw_err;  // [0] failed, [1] system index (q position x nw_b + Omega), [2] info
-  int gw_err_host[3] = {0, 0, 0};
+  int* gw_err_host = nullptr;       // gw_err in pinned host memory, there once dyson_done has passed (eager builds)
+  cudaEvent_t dyson_done = nullptr;
+  int* dyson_status() {
+    if (!gw_err_host) GG_CUDA(cudaMallocHost((void**)&gw_err_host, 3 * sizeof(int)));
+    if (!dyson_done) GG_CUDA(cudaEventCreateWithFlags(&dyson_done, cudaEventDisableTiming));
+    return gw_err_host;
+  }
   // plan of the last eager build (plan_key: precision, spin blocks and solver), reused by later ones and by the capture
   gg::Plan plan;
   int plan_key = -1;
@@ -161,6 +167,8 @@ struct gg_context {
   ~gg_context() {
     drop_graph();
     for (auto ev : events) cudaEventDestroy(ev);
+    if (dyson_done) cudaEventDestroy(dyson_done);
+    if (gw_err_host) cudaFreeHost(gw_err_host);
     if (split) gg::split_release(split);
     if (stream) cudaStreamDestroy(stream);
   }

@@ -669,10 +669,16 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
       c->launches += launch_dyson(Pw + (long)s0 * NN, Af, lu_inv, info + s0, sn, N, solver, piv, st);
     }
     tm.end(h);
-    // no host round trip in the middle of a build: the first failing system is recorded on the device
-    // and reported at the end
+    // the first failing system is recorded on the device.  A graph replay reports it at its end; an eager build reads it
+    // once the first star member's Sigma is in the queue behind it, so that a failure does not cost the whole
+    // Sigma phase and the wait leaves the GPU with work
     launch_info_collect(info, qn * nw, q0 * nw, gw_err, st);
     ++c->launches;
+    bool dyson_read = cap;
+    if (!cap) {
+      GG_CUDA(cudaMemcpyAsync(c->dyson_status(), gw_err, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
+      GG_CUDA(cudaEventRecord(c->dyson_done, st));
+    }
     // ---------------- IR back: Wt[q][t] = sum_w Ttn[t][w] W[q][w]
     h = tm.begin(5);
     {
@@ -799,16 +805,23 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
             }
           }
         }
+        if (!dyson_read) {
+          dyson_read = true;
+          GG_CUDA(cudaEventSynchronize(c->dyson_done));
+          const int* e = c->dyson_status();
+          if (e[0]) {
+            GG_CUDA(cudaStreamSynchronize(st));  // nothing of a failed build is left running
+            dyson_failure(c, solver, e[1], e[2]);
+          }
+        }
       }
     }
     tm.end(h);
   }
   tm.end(h_total);
   if (cap) return;  // the caller checks gw_err and the split engine's flag after the replay
-  GG_CUDA(cudaMemcpyAsync(c->gw_err_host, gw_err, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
   if (split) split_check(split, st);
   GG_CUDA(cudaStreamSynchronize(st));
-  if (c->gw_err_host[0]) dyson_failure(c, solver, c->gw_err_host[1], c->gw_err_host[2]);
   for (auto& e : kev) {
     float ms = 0;
     GG_CUDA(cudaEventElapsedTime(&ms, e.second.first, e.second.second));
