@@ -182,10 +182,10 @@ int zgemm(const ZgemmDesc& d0, cudaStream_t stream) {
   // anyway, and CTAs of one team drift apart by themselves)
   const double tile_ns = (double)groups / d.splits * s.mt * s.nt * (d.gauss ? 3 : 4) * 16.0 * s.warps / 4 / 1.9;
   g.stagger = items >= 4 * teams && tile_ns < 200e3 ? (int)tile_ns : 0;
-  if (ak && bk) zgemm_launch_kk(ch.shape, d.gauss != 0, d, g, teams, stream);
-  else if (ak) zgemm_launch_kn(ch.shape, d.gauss != 0, d, g, teams, stream);
-  else if (bk) zgemm_launch_nk(ch.shape, d, g, teams, stream);
-  else zgemm_launch_nn(ch.shape, d, g, teams, stream);
+  if (ak && bk) zgemm_launch_kk(ch.shape, d.gauss != 0, d, g, stream);
+  else if (ak) zgemm_launch_kn(ch.shape, d.gauss != 0, d, g, stream);
+  else if (bk) zgemm_launch_nk(ch.shape, d, g, stream);
+  else zgemm_launch_nn(ch.shape, d, g, stream);
   int launches = 1;
   if (d.splits > 1) {
     const long total = (long)d.M * d.N * batch;

@@ -534,19 +534,25 @@ template <> struct ZTileOf<9, true> { using T = ZTile<2, 2, 2, 2, 3, 5, 1>; };
 template <> struct ZTileOf<10, true> { using T = ZTile<1, 1, 2, 2, 4, 7, 2>; };
 
 // launch shape `shape` of one layout (G3 where the layout has it)
-void zgemm_launch_kk(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st);
-void zgemm_launch_kn(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st);
-void zgemm_launch_nk(int shape, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st);
-void zgemm_launch_nn(int shape, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st);
+void zgemm_launch_kk(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, cudaStream_t st);
+void zgemm_launch_kn(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, cudaStream_t st);
+void zgemm_launch_nk(int shape, const ZgemmDesc& d, const ZGrid& g, cudaStream_t st);
+void zgemm_launch_nn(int shape, const ZgemmDesc& d, const ZGrid& g, cudaStream_t st);
 // products that do not fill the GPU, any layout: one CTA per 8 x 8 tile (zgemm_small.cu)
 void zgemm_launch_small(const ZgemmDesc& d, const ZGrid& g, cudaStream_t st);
 
+// CTAs for `items` tiles with `resident` teams per SM.  Paired: one CTA per SM as long as there are items, so that no SM's
+// second team gets one before every SM has its first.  Unpaired: up to four rounds of items go out as a CTA each, which
+// the hardware deals to SMs as they become free (a fixed assignment gives SMs whose CTAs all have one
+// item more than others: 160 x 160 x 3200, batch 12: 0.33 against 0.27 ms), more as persistent CTAs.
+inline long zgemm_ctas(long items, long sms, int resident, bool pair) {
+  if (pair) return items < sms ? items : sms;
+  const long teams = sms * resident;
+  return items <= 4 * teams ? items : teams;
+}
+
 template <class T, bool A_K, bool B_K, bool G3>
-void zlaunch(const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st) {
-  // up to four rounds of items go out as a CTA each, which the hardware deals to SMs as they become free: a
-  // fixed assignment gives SMs whose CTAs all have one item more than others (160 x 160 x 3200, batch 12: 0.33
-  // against 0.27 ms)
-  if (!T::PAIR && g.items <= 4 * teams) teams = g.items;
+void zlaunch(const ZgemmDesc& d, const ZGrid& g, cudaStream_t st) {
   // the shared-memory attribute is per device: set once on each
   static std::atomic<bool> cfg[kMaxDevices];
   const int dev = current_device();
@@ -554,20 +560,21 @@ void zlaunch(const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st) {
     GG_CUDA(cudaFuncSetAttribute(zgemm_kernel<T, A_K, B_K, G3>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM));
     cfg[dev].store(true, std::memory_order_release);
   }
-  zgemm_kernel<T, A_K, B_K, G3><<<(unsigned)((teams + T::TEAMS - 1) / T::TEAMS), T::THREADS, T::SMEM, st>>>(d, g);
+  const unsigned ctas = (unsigned)zgemm_ctas(g.items, device_sm_count(), T::TEAMS * T::MINB, T::PAIR);
+  zgemm_kernel<T, A_K, B_K, G3><<<ctas, T::THREADS, T::SMEM, st>>>(d, g);
   GG_CHECK_LAUNCH();
 }
 
 template <bool A_K, bool B_K, bool G3, int I = 0>
-void zlaunch_shape(int shape, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st) {
+void zlaunch_shape(int shape, const ZgemmDesc& d, const ZGrid& g, cudaStream_t st) {
   if constexpr (I < (G3 ? kZShapes3 : kZShapes)) {
     using T = typename ZTileOf<I, G3>::T;
     constexpr ZShape s = G3 ? kZShape3[I < kZShapes3 ? I : 0] : kZShape[I];
     static_assert(T::BM == s.bm && T::BN == s.bn && T::MT == s.mt && T::NT == s.nt && T::WARPS == s.warps &&
                       T::TEAMS * T::MINB == s.teams,
                   "shape table");
-    if (shape == I) zlaunch<T, A_K, B_K, G3>(d, g, teams, st);
-    else zlaunch_shape<A_K, B_K, G3, I + 1>(shape, d, g, teams, st);
+    if (shape == I) zlaunch<T, A_K, B_K, G3>(d, g, st);
+    else zlaunch_shape<A_K, B_K, G3, I + 1>(shape, d, g, st);
   }
 }
 

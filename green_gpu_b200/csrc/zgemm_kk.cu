@@ -5,9 +5,9 @@
 
 namespace gg {
 
-void zgemm_launch_kk(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st) {
-  if (g3) zlaunch_shape<true, true, true>(shape, d, g, teams, st);
-  else zlaunch_shape<true, true, false>(shape, d, g, teams, st);
+void zgemm_launch_kk(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, cudaStream_t st) {
+  if (g3) zlaunch_shape<true, true, true>(shape, d, g, st);
+  else zlaunch_shape<true, true, false>(shape, d, g, st);
 }
 
 }  // namespace gg

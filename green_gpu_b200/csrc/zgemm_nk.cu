@@ -5,8 +5,8 @@
 
 namespace gg {
 
-void zgemm_launch_nk(int shape, const ZgemmDesc& d, const ZGrid& g, long teams, cudaStream_t st) {
-  zlaunch_shape<false, true, false>(shape, d, g, teams, st);
+void zgemm_launch_nk(int shape, const ZgemmDesc& d, const ZGrid& g, cudaStream_t st) {
+  zlaunch_shape<false, true, false>(shape, d, g, st);
 }
 
 }  // namespace gg

@@ -1,7 +1,8 @@
 // Internal functions of libgreen_b200.so behind plain C calls, for the tests that look at them directly.
-#include <cstring>
+#include <atomic>
 
 #include "engine.cuh"
+#include "zgemm_kernel.cuh"
 
 // out: q points, k points, tau points, Dyson systems per chunk, bytes; returns the error code of a refused shape
 extern "C" int plan_work(const gg_shape* s, int nspin, int slices, int solver, int64_t budget, int64_t* out) {
@@ -16,4 +17,8 @@ extern "C" int plan_work(const gg_shape* s, int nspin, int slices, int solver, i
   } catch (const gg::Error& e) {
     return e.code;
   }
+}
+
+extern "C" int64_t zgemm_ctas(int64_t items, int64_t sms, int resident, int pair) {
+  return gg::zgemm_ctas(items, sms, resident, pair != 0);
 }
