@@ -136,10 +136,11 @@ struct gg_context {
   std::vector<const void*> graph_sig;
   gg::DevBuf<int> gw_flag;  // nonzero: this build's G is Hermitian
   gg::DevBuf<int> gw_err;  // [0] failed, [1] system index (q position x nw_b + Omega), [2] info
-  int* gw_err_host = nullptr;       // gw_err in pinned host memory, there once dyson_done has passed (eager builds)
+  // pinned host memory of eager builds: gw_err, there once dyson_done has passed, and gw_flag, there at the end
+  int* gw_err_host = nullptr;
   cudaEvent_t dyson_done = nullptr;
   int* dyson_status() {
-    if (!gw_err_host) GG_CUDA(cudaMallocHost((void**)&gw_err_host, 3 * sizeof(int)));
+    if (!gw_err_host) GG_CUDA(cudaMallocHost((void**)&gw_err_host, 4 * sizeof(int)));
     if (!dyson_done) GG_CUDA(cudaEventCreateWithFlags(&dyson_done, cudaEventDisableTiming));
     return gw_err_host;
   }

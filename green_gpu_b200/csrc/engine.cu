@@ -820,8 +820,12 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
   }
   tm.end(h_total);
   if (cap) return;  // the caller checks gw_err and the split engine's flag after the replay
+  int* herm_h = c->dyson_status() + 3;
+  if (herm) GG_CUDA(cudaMemcpyAsync(herm_h, herm, sizeof(int), cudaMemcpyDeviceToHost, st));
   if (split) split_check(split, st);
   GG_CUDA(cudaStreamSynchronize(st));
+  // the lower triangle with its diagonal is what a P0 product did and needed
+  if (herm && *herm_h) c->kstat_flops[0] *= (N + 1.0) / (2.0 * N);
   for (auto& e : kev) {
     float ms = 0;
     GG_CUDA(cudaEventElapsedTime(&ms, e.second.first, e.second.second));

@@ -210,7 +210,8 @@ int gg_last_timings(const gg_context* ctx, double* out, int n);
  * gg_set_fused_tail the fused kernel that also forms its operand Z = X G.  Each entry covers
  * launches of one kernel kind.
  * Writes launches, total seconds and algorithmic flops
- * (8MNK + 12MN per complex GEMM, src/green/gpu/common_defs.h:121-125). */
+ * (8MNK + 12MN per complex GEMM, src/green/gpu/common_defs.h:121-125; N (N + 1) / 2 of the N^2 elements where an
+ * FP64 build computes only the lower triangle of P0, for Hermitian G). */
 int gg_set_profiling(gg_context* ctx, int enable);
 int gg_kernel_stats(const gg_context* ctx, int which, int64_t* launches, double* seconds, double* flops);
 /* Number of kernel launches issued by the last GW build or HF call. */
