@@ -286,7 +286,7 @@ std::vector<const void*> gg_context::buffer_signature() const {
                                 Tnt_fold.p, x2c_in.p, x2c_out.p, G_in.p, Sigma_out.p, Gf.p,       Gtmp.p,
                                 Vbuf.p,  G1buf.p,   scratchA.p, scratchB.p, P0buf.p, Pw.p,     Afac.p,
                                 Wt.p,    Wrot.p,    gemm_work.p, hf_D.p,  hf_F.p,      hf_c.p,     hf_J.p,  hf_S.p,
-                                info.p,  piv.p,     idx_i.p,   pos_d.p,  op_d.p,      gw_err.p,   gw_tables.get(),
+                                info.p,  piv.p,     gw_err.p,   gw_tables.get(),
                                 p0_ea.p, p0_eb.p,    lu_inv.p,   gw_flag.p};
   split_buffers(split, v);
   return v;

@@ -67,7 +67,6 @@ struct gg_context {
   std::vector<std::vector<int>> k_stars, q_stars;
   bool has_Uk = false, has_Uq = false;
   gg::DevBuf<double2> Uk, Uq;
-  std::vector<double2> Uk_h;
   gg::DevBuf<int> k_f2r_d, k_tr_d;
 
   // k-pair store
@@ -101,12 +100,10 @@ struct gg_context {
   // work buffers
   gg::DevBuf<double2> G_in, Sigma_out, Gf, Gtmp, Vbuf, G1buf, scratchA, scratchB, P0buf, Pw, Afac, Wt, Wrot,
       gemm_work, hf_D, hf_F, hf_c, hf_J, hf_S, lu_inv;
-  gg::DevBuf<int> info, piv, idx_i;
+  gg::DevBuf<int> info, piv;
   // split precision: exponents of the P0 main contraction's operand rows / columns, recorded
   // by the operand builds' epilogues
   gg::DevBuf<int> p0_ea, p0_eb;
-  gg::DevBuf<int64_t> pos_d;
-  gg::DevBuf<int> op_d;
 
   gg::Timings last{};
   long launches = 0;

@@ -96,11 +96,6 @@ __global__ void transpose_blocks_kernel(const double2* __restrict__ in, int n, i
   }
 }
 
-__global__ void scale_kernel(double2* X, long n, double s) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-    X[i] = cscale(X[i], s);
-}
-
 // One CTA per matrix (blockIdx.x = (t * ns + s) * ink + k): clears *flag unless G[t][s][k] and G[t][s'][k]^H agree
 // within tol of the largest element of either, s' = s or, with `swap` (X2C spin blocks), 0, 1, 3, 2
 __global__ void __launch_bounds__(128) hermitian_check_kernel(const double2* __restrict__ G, int ns, int ink, int n, int swap,
@@ -390,15 +385,6 @@ void launch_mirror_lower(double2* X, int nmat, int n, const int* flag, cudaStrea
   const int t = ceil_div(n, 32);
   mirror_lower_kernel<<<(unsigned)((long)nmat * t * (t + 1) / 2), TPB, 0, st>>>(X, nmat, n, flag);
   GG_CHECK_LAUNCH();
-}
-
-void launch_scale(double2* X, long n, double s, cudaStream_t st) {
-  scale_kernel<<<grid_for(n), TPB, 0, st>>>(X, n, s);
-  GG_CHECK_LAUNCH();
-}
-
-void launch_fill_zero(double2* X, long n, cudaStream_t st) {
-  GG_CUDA(cudaMemsetAsync(X, 0, sizeof(double2) * n, st));
 }
 
 void launch_hartree_coeff(const double2* S, const int64_t* pos_d, const int* op_d, const double2* D, int nk, int NQ, int n,

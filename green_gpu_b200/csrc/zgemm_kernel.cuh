@@ -498,9 +498,8 @@ constexpr ZShape kZShape[] = {
     {56, 56, 1, 7, 7, 2}, {48, 48, 1, 6, 6, 2}, {40, 40, 1, 5, 5, 3}, {24, 24, 1, 3, 3, 4}, {32, 32, 2, 2, 4, 3},
     {16, 16, 1, 1, 4, 4}};
 constexpr ZShape kZShape3[] = {
-    {64, 48, 4, 3, 4, 2}, {64, 56, 2, 7, 4, 2}, {64, 48, 2, 6, 4, 2}, {64, 40, 2, 5, 4, 2}, {64, 32, 2, 4, 4, 2},
-    {64, 24, 2, 3, 4, 3}, {64, 16, 2, 2, 4, 3}, {64, 8, 2, 1, 4, 4}, {32, 56, 1, 7, 4, 3}, {32, 32, 2, 2, 4, 3},
-    {16, 16, 1, 1, 4, 4}};
+    {64, 48, 4, 3, 4, 2}, {64, 56, 2, 7, 4, 2}, {64, 40, 2, 5, 4, 2}, {64, 32, 2, 4, 4, 2}, {64, 24, 2, 3, 4, 3},
+    {64, 16, 2, 2, 4, 3}, {64, 8, 2, 1, 4, 4},  {32, 56, 1, 7, 4, 3}, {32, 32, 2, 2, 4, 3}, {16, 16, 1, 1, 4, 4}};
 constexpr int kZShapes = sizeof(kZShape) / sizeof(ZShape), kZShapes3 = sizeof(kZShape3) / sizeof(ZShape);
 
 template <int I, bool G3>
@@ -523,15 +522,14 @@ template <> struct ZTileOf<14, false> { using T = ZTile<2, 2, 2, 2, 3, 5, 1>; };
 template <> struct ZTileOf<15, false> { using T = ZTile<1, 1, 2, 2, 4, 7, 2>; };
 template <> struct ZTileOf<0, true> { using T = ZTile<4, 3, 2, 2, 1, 3, 1, true>; };
 template <> struct ZTileOf<1, true> { using T = ZTile<2, 7, 4, 1, 1, 3, 1, true>; };
-template <> struct ZTileOf<2, true> { using T = ZTile<2, 6, 4, 1, 1, 3, 1, true>; };
-template <> struct ZTileOf<3, true> { using T = ZTile<2, 5, 4, 1, 1, 3, 1, true>; };
-template <> struct ZTileOf<4, true> { using T = ZTile<2, 4, 4, 1, 1, 3, 1, true>; };
-template <> struct ZTileOf<5, true> { using T = ZTile<2, 3, 4, 1, 3, 4, 1>; };
-template <> struct ZTileOf<6, true> { using T = ZTile<2, 2, 4, 1, 3, 4, 1>; };
-template <> struct ZTileOf<7, true> { using T = ZTile<2, 1, 4, 1, 4, 5, 2>; };
-template <> struct ZTileOf<8, true> { using T = ZTile<1, 7, 4, 1, 3, 4, 1>; };
-template <> struct ZTileOf<9, true> { using T = ZTile<2, 2, 2, 2, 3, 5, 1>; };
-template <> struct ZTileOf<10, true> { using T = ZTile<1, 1, 2, 2, 4, 7, 2>; };
+template <> struct ZTileOf<2, true> { using T = ZTile<2, 5, 4, 1, 1, 3, 1, true>; };
+template <> struct ZTileOf<3, true> { using T = ZTile<2, 4, 4, 1, 1, 3, 1, true>; };
+template <> struct ZTileOf<4, true> { using T = ZTile<2, 3, 4, 1, 3, 4, 1>; };
+template <> struct ZTileOf<5, true> { using T = ZTile<2, 2, 4, 1, 3, 4, 1>; };
+template <> struct ZTileOf<6, true> { using T = ZTile<2, 1, 4, 1, 4, 5, 2>; };
+template <> struct ZTileOf<7, true> { using T = ZTile<1, 7, 4, 1, 3, 4, 1>; };
+template <> struct ZTileOf<8, true> { using T = ZTile<2, 2, 2, 2, 3, 5, 1>; };
+template <> struct ZTileOf<9, true> { using T = ZTile<1, 1, 2, 2, 4, 7, 2>; };
 
 // launch shape `shape` of one layout (G3 where the layout has it)
 void zgemm_launch_kk(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, cudaStream_t st);
