@@ -48,7 +48,6 @@ void launch_hermitian_part(const double2* G, int nk, int ns, int nts, int n, int
 // where *flag (device): the upper triangles of nmat n x n matrices from their lower ones
 void launch_mirror_lower(double2* X, int nmat, int n, const int* flag, cudaStream_t st);
 
-
 // Batched Dyson solve for `nsys` systems of size N x N stored contiguously in P (in place):
 // P <- Hermitian-symmetrise(P); A = I - P; Cholesky: P <- (A^{-1} P)^H, LU: P <- sym(A^{-1} P).
 // `A` is a workspace of the same size, `info` receives per-system status (0 ok; Cholesky:

@@ -146,27 +146,37 @@ int zgemm(const ZgemmDesc& d0, cudaStream_t stream) {
   if (d.K < 0 || d.KB < 1) throw Error(GG_ERR_ARG, "zgemm: bad K");
   if (d.tri && d.M != d.N) throw Error(GG_ERR_INTERNAL, "zgemm: the lower triangle of a product that is not square");
   const long batch = (long)d.nb0 * d.nb1 * d.nb2;
-  ZGrid g = {};
-  g.gpb = std::max(1, ceil_div(d.K, 4));
-  const long groups = (long)d.KB * g.gpb;
+  const int gpb = std::max(1, ceil_div(d.K, 4));
+  const long groups = (long)d.KB * gpb;
   const int sms = device_sm_count();
   // one round of 8 x 8 tiles (four CTAs per SM) with at most 24 groups per warp: the latency-bound kernel (beyond
   // it the staged tiles win: eight of 100^3 10.6 against 13.3 us)
   const long tiles8 = (long)ceil_div(d.M, 8) * ceil_div(d.N, 8) * batch;
   if (tiles8 <= 4L * sms && groups <= 96 && !d.tri && !d.inplace) {
-    d.splits = 1;
+    ZGrid g = {};
+    g.gpb = gpb;
     g.tiles_m = ceil_div(d.M, 8);
     g.tiles_n = ceil_div(d.N, 8);
     g.items = (int)tiles8;
     g.groups = (int)groups;
+    d.splits = 1;
     zgemm_launch_small(d, g, stream);
     return 1;
   }
-  const bool ak = (d.a_k == 1), bk = (d.b_k == 1);
-  if (!ak) d.gauss = 0;  // the three-product kernels exist where split builds use them (k-contiguous A)
+  if (d.a_k != 1) d.gauss = 0;  // the three-product kernels exist where split builds use them (k-contiguous A)
   const ZChoice ch = choose(d, batch, groups, sms);
-  const ZShape& s = d.gauss ? kZShape3[ch.shape] : kZShape[ch.shape];
   d.splits = ch.splits;
+  return zgemm_shape(d, ch.shape, stream);
+}
+
+int zgemm_shape(const ZgemmDesc& d, int shape, cudaStream_t stream) {
+  const bool ak = (d.a_k == 1), bk = (d.b_k == 1);
+  const ZShape& s = d.gauss ? kZShape3[shape] : kZShape[shape];
+  const long batch = (long)d.nb0 * d.nb1 * d.nb2;
+  const int sms = device_sm_count();
+  ZGrid g = {};
+  g.gpb = std::max(1, ceil_div(d.K, 4));
+  const long groups = (long)d.KB * g.gpb;
   g.tiles_m = ceil_div(d.M, s.bm);
   g.tiles_n = ceil_div(d.N, s.bn);
   g.tri_tiles = tri_tiles(g.tiles_m, g.tiles_n, s.bm, s.bn);
@@ -182,10 +192,10 @@ int zgemm(const ZgemmDesc& d0, cudaStream_t stream) {
   // anyway, and CTAs of one team drift apart by themselves)
   const double tile_ns = (double)groups / d.splits * s.mt * s.nt * (d.gauss ? 3 : 4) * 16.0 * s.warps / 4 / 1.9;
   g.stagger = items >= 4 * teams && tile_ns < 200e3 ? (int)tile_ns : 0;
-  if (ak && bk) zgemm_launch_kk(ch.shape, d.gauss != 0, d, g, stream);
-  else if (ak) zgemm_launch_kn(ch.shape, d.gauss != 0, d, g, stream);
-  else if (bk) zgemm_launch_nk(ch.shape, d, g, stream);
-  else zgemm_launch_nn(ch.shape, d, g, stream);
+  if (ak && bk) zgemm_launch_kk(shape, d.gauss != 0, d, g, stream);
+  else if (ak) zgemm_launch_kn(shape, d.gauss != 0, d, g, stream);
+  else if (bk) zgemm_launch_nk(shape, d, g, stream);
+  else zgemm_launch_nn(shape, d, g, stream);
   int launches = 1;
   if (d.splits > 1) {
     const long total = (long)d.M * d.N * batch;

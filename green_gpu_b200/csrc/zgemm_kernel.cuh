@@ -531,6 +531,9 @@ template <> struct ZTileOf<7, true> { using T = ZTile<1, 7, 4, 1, 3, 4, 1>; };
 template <> struct ZTileOf<8, true> { using T = ZTile<2, 2, 2, 2, 3, 5, 1>; };
 template <> struct ZTileOf<9, true> { using T = ZTile<1, 1, 2, 2, 4, 7, 2>; };
 
+// the product with shape `shape` of the table (three products: of kZShape3) and d.splits partial sums, the pass over
+// which follows; returns the launches (zgemm.cu)
+int zgemm_shape(const ZgemmDesc& d, int shape, cudaStream_t stream);
 // launch shape `shape` of one layout (G3 where the layout has it)
 void zgemm_launch_kk(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, cudaStream_t st);
 void zgemm_launch_kn(int shape, bool g3, const ZgemmDesc& d, const ZGrid& g, cudaStream_t st);
