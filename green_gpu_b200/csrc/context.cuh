@@ -131,10 +131,9 @@ struct gg_context {
   // device addresses of every work buffer when the graph was captured: an entry point that
   // grows a shared buffer (HF, unfold, zgemm) reallocates it, and the graph is then rebuilt
   std::vector<const void*> graph_sig;
-  gg::DevBuf<int> gw_flag;  // nonzero: this build's G is Hermitian
-  gg::DevBuf<int> gw_err;  // [0] failed, [1] system index (q position x nw_b + Omega), [2] info
-  // pinned host memory of eager builds: gw_err, there once dyson_done has passed, and gw_flag, there at the end
-  int* gw_err_host = nullptr;
+  // [0] failed, [1] system index (q position x nw_b + Omega), [2] info, [3] nonzero: this (FP64) build's G is Hermitian
+  gg::DevBuf<int> gw_err;
+  int* gw_err_host = nullptr;  // the same in pinned host memory, there once dyson_done has passed (eager builds)
   cudaEvent_t dyson_done = nullptr;
   int* dyson_status() {
     if (!gw_err_host) GG_CUDA(cudaMallocHost((void**)&gw_err_host, 4 * sizeof(int)));

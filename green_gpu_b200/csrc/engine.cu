@@ -541,7 +541,7 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
   // (Sigma 8.3e-10 instead of 5.9e-10 from the lower triangle alone).
   int* herm = nullptr;
   if (!split) {
-    herm = c->gw_flag.ensure(1);
+    herm = gw_err + 3;
     launch_hermitian_check(G_dev, T, ns, s.ink, n, c->x2c, c->cap_P0 ? 0x1p-49 : 0x1p-46, herm, st);
     ++c->launches;
   }
@@ -676,7 +676,7 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
     ++c->launches;
     bool dyson_read = cap;
     if (!cap) {
-      GG_CUDA(cudaMemcpyAsync(c->dyson_status(), gw_err, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
+      GG_CUDA(cudaMemcpyAsync(c->dyson_status(), gw_err, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
       GG_CUDA(cudaEventRecord(c->dyson_done, st));
     }
     // ---------------- IR back: Wt[q][t] = sum_w Ttn[t][w] W[q][w]
@@ -820,12 +820,10 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
   }
   tm.end(h_total);
   if (cap) return;  // the caller checks gw_err and the split engine's flag after the replay
-  int* herm_h = c->dyson_status() + 3;
-  if (herm) GG_CUDA(cudaMemcpyAsync(herm_h, herm, sizeof(int), cudaMemcpyDeviceToHost, st));
   if (split) split_check(split, st);
   GG_CUDA(cudaStreamSynchronize(st));
   // the lower triangle with its diagonal is what a P0 product did and needed
-  if (herm && *herm_h) c->kstat_flops[0] *= (N + 1.0) / (2.0 * N);
+  if (herm && nmy > 0 && c->dyson_status()[3]) c->kstat_flops[0] *= (N + 1.0) / (2.0 * N);
   for (auto& e : kev) {
     float ms = 0;
     GG_CUDA(cudaEventElapsedTime(&ms, e.second.first, e.second.second));
