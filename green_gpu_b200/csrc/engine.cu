@@ -301,8 +301,11 @@ ZgemmDesc transposed(const ZgemmDesc& d) {
   return t;
 }
 
-// P0 of one k chunk (kn points from k0) and one spin in split precision.  The operand builds
-// (INT8 engine, FP64 output SA / SB as in the FP64 path) also record the exact maximum of every
+// P0 of one k chunk (kn points from k0) and one spin in split precision.  The O(nao^3 NQ) operand builds (G V and V^+ G)
+// run on the INT8 engine too: their large operand V is sliced once per launch for the whole tau block and G is
+// small, so at nao 52 slicing costs little next to the FP64 GEMM it replaces.  For small nao that is not
+// settled: at nao 26 a build takes 88 us after slicing, and 86 to 92 us on the FP64 engine (four products).
+// The builds (FP64 output SA / SB as in the FP64 path) also record the exact maximum of every
 // row of SA and every column of SB that the main contraction slices with (a segmented warp
 // reduction and one atomicMax per row segment in their epilogue), so the two exponent scans over
 // SA and SB - a full read of both - are not needed; the slicing pass uses those exponents.
@@ -471,23 +474,6 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
     }
   };
 
-  // the O(nao^3 NQ) operand builds of P0 (G V and V^+ G) also run on the INT8 engine in split
-  // precision: their large operand V is sliced once per launch for the whole tau block and
-  // the G operand is small, so slicing costs little next to the FP64 GEMM it replaces
-  // The INT8 engine's epilogue gives each lane one row of C, so its stores coalesce when C is
-  // contiguous along m; the build outputs are contiguous along n, so they are computed as
-  // C^T = B^T A^T (the same slices and int32 sums, so the same result).
-  auto gemm_build = [&](ZgemmDesc d) {
-    if (split) {
-      ZgemmDesc t = transposed(d);
-      t.work = gw_work;
-      t.work_elems = (long)c->gemm_work.n;
-      c->launches += split_zgemm(split, t, c->slices, st);
-    } else {
-      gemm(d);
-    }
-  };
-
   // pair tables: P0 pairs (k, k+q) for every irreducible q, Sigma pairs (k_ibz, k_ibz - q');
   // G1 block indices: block (k1 * ns + sp) of Gf, for every (iq, sp, k).  Built once per
   // symmetry / k-pair / spin setting (the uploads synchronise, so never while capturing).
@@ -597,7 +583,7 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
               d.c_n.split = n; d.c_n.hi = nn; d.c_n.lo = 1;
               d.nb0 = kn;
               d.a_b0 = (long)ns * T * nn; d.b_b0 = Nnn; d.c_b0 = (long)tn * Nnn;
-              gemm_build(d);
+              gemm(d);
             }
             // B-build: SB[kk][tt][Q][a][b] = sum_l conj(V[kk][Q][a][l]) G^{k+q}(tau_t)[b][l],
             // tau folded into the columns, n = (tt, b)
@@ -609,7 +595,7 @@ void gw_build(gg_context* c, const double2* G_dev, double2* Sigma_dev, int solve
               d.C = SB; d.c_m.lo = n; d.c_n.split = n; d.c_n.hi = Nnn; d.c_n.lo = 1;
               d.nb0 = kn;
               d.a_b0 = Nnn; d.b_b0 = (long)T2 * nn; d.c_b0 = (long)tn * Nnn;
-              gemm_build(d);
+              gemm(d);
             }
             // P0[q][t] (+)= pref/nk sum_kk sum_x SA[kk][tt][Q'][x] SB[kk][tt][Q][x]
             {
