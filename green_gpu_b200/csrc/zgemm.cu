@@ -56,10 +56,22 @@ int tri_tiles(int tiles_m, int tiles_n, int bm, int bn) {
   return count;
 }
 
-// Tile shape and split-K factor of a descriptor.
-struct ZChoice {
-  int shape = 0, splits = 1;
-};
+// Least split-K factor.  The rounding error of a sum grows with its length (120 x 120 x 5408: 2.7e-15 as one sum, 6.7e-16
+// as four), so a four-product sum is cut until an accumulator adds up at most 128 groups, as far as the parts leave at
+// most four 64 x 64 tiles per SM, 256 parts and room for them: beyond that the pass over the parts
+// costs more (exchange of the Fock build 5.3 -> 5.5 ms with 547 parts instead of 296).  By time alone small tiles, which fill
+// the GPU with few parts, have long sums: Sigma of nao 26, NQ 120 (P0 in 4 parts, now 11) was off by 5.3 to 8.4e-15 and is by
+// 2.2 to 2.9e-15, of nao 36, NQ 250 (1 part, now 4) 3.3e-15 and 9.5e-16.  It costs 0 to 2 % of a build (spinors of
+// 2 x 26 10.82 -> 10.92 ms; nao 26, NQ 120 33.9 -> 33.7).
+long least_splits(const ZgemmDesc& d, long batch, long groups, int sms) {
+  if (d.gauss || d.inplace || !d.work) return 1;
+  const double out = (double)d.M * d.N * batch;
+  const long tiles64 = (long)ceil_div(d.M, 64) * ceil_div(d.N, 64) * batch;
+  const long parts = std::min(std::min((groups + 127) / 128, (4L * sms + tiles64 - 1) / tiles64), 256L);
+  return std::max(1L, std::min(parts, std::min(groups / 8, (long)((double)d.work_elems / out))));
+}
+
+}  // namespace
 
 // The choice minimises a cycle estimate fitted to timings of every shape and split on 33 of the
 // library's products (outputs of 20..400 columns, reductions of 20..280000, batches of 1..72; the chosen
@@ -74,12 +86,13 @@ struct ZChoice {
 //          of 16 x 16, 17.3 us on one of 64 x 64);
 //   l2     operand tiles arrive at about 40 bytes per cycle and SM.
 // Splitting the reduction multiplies the tiles and adds a launch and the pass over the partial sums.
-ZChoice choose(const ZgemmDesc& d, long batch, long groups, int sms) {
+ZChoice zgemm_choose(const ZgemmDesc& d, long batch, long groups, int sms) {
   static const int kSplits[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 48, 64, 96, 128, 192, 256, 384, 512};
   const ZShape* const table = d.gauss ? kZShape3 : kZShape;
   const int count = d.gauss ? kZShapes3 : kZShapes;
   const double prods = d.gauss ? 3.0 : 4.0;
   const double out = (double)d.M * d.N * batch;
+  const int least = (int)least_splits(d, batch, groups, sms);
   ZChoice best;
   double best_cost = 0.0;
   bool have = false;
@@ -93,6 +106,7 @@ ZChoice choose(const ZgemmDesc& d, long batch, long groups, int sms) {
         (0.89 - 0.5 / t88) * (d.gauss ? 0.8 : 1.0) * (s.square() ? 0.9 : 1.0);
     const double group = std::max(1.15 * mma + 100.0, 150.0 + 7.0 * (s.bm + s.bn));
     auto consider = [&](int sp) {
+      if (sp < least) return;
       if (sp > 1 && (d.inplace || !d.work || groups / sp < 8 || out * sp > (double)d.work_elems)) return;
       const double g = (double)((groups + sp - 1) / sp), items = tiles * sp;
       const double per_sm = std::ceil(items / sms), waves = std::ceil(items / ((double)sms * s.teams));
@@ -109,6 +123,7 @@ ZChoice choose(const ZgemmDesc& d, long batch, long groups, int sms) {
       }
     };
     for (int sp : kSplits) consider(sp);
+    consider(least);
     // splits that fill whole rounds of SMs: with 256 of them over 148 SMs, 40 SMs have one CTA and the others two
     // (36 x 36 x 279936: 194 us, 171 us with 296; Z V^+ of nao 37, three products: 0.252 -> 0.229 ms)
     for (int r = 1; r <= 4; ++r) {
@@ -119,8 +134,6 @@ ZChoice choose(const ZgemmDesc& d, long batch, long groups, int sms) {
   if (!have) throw Error(GG_ERR_INTERNAL, "zgemm: no tile shape for an in-place product of this size");
   return best;
 }
-
-}  // namespace
 
 int current_device() {
   int dev = 0;
@@ -164,7 +177,7 @@ int zgemm(const ZgemmDesc& d0, cudaStream_t stream) {
     return 1;
   }
   if (d.a_k != 1) d.gauss = 0;  // the three-product kernels exist where split builds use them (k-contiguous A)
-  const ZChoice ch = choose(d, batch, groups, sms);
+  const ZChoice ch = zgemm_choose(d, batch, groups, sms);
   d.splits = ch.splits;
   return zgemm_shape(d, ch.shape, stream);
 }

@@ -531,6 +531,11 @@ template <> struct ZTileOf<7, true> { using T = ZTile<1, 7, 4, 1, 3, 4, 1>; };
 template <> struct ZTileOf<8, true> { using T = ZTile<2, 2, 2, 2, 3, 5, 1>; };
 template <> struct ZTileOf<9, true> { using T = ZTile<1, 1, 2, 2, 4, 7, 2>; };
 
+// tile shape and split-K factor of a descriptor on a GPU of `sms` SMs (zgemm.cu)
+struct ZChoice {
+  int shape = 0, splits = 1;
+};
+ZChoice zgemm_choose(const ZgemmDesc& d, long batch, long groups, int sms);
 // the product with shape `shape` of the table (three products: of kZShape3) and d.splits partial sums, the pass over
 // which follows; returns the launches (zgemm.cu)
 int zgemm_shape(const ZgemmDesc& d, int shape, cudaStream_t stream);

@@ -23,6 +23,17 @@ extern "C" int64_t zgemm_ctas(int64_t items, int64_t sms, int resident, int pair
   return gg::zgemm_ctas(items, sms, resident, pair != 0);
 }
 
+// split factor chosen for `batch` products of M x N x (KB K) with room for `room` partial sums
+extern "C" int zgemm_splits(int M, int N, int K, int KB, int batch, int tri, int gauss, int64_t room, int sms) {
+  static int flag;
+  gg::ZgemmDesc d;
+  d.M = M; d.N = N; d.K = K; d.KB = KB; d.nb0 = batch; d.gauss = gauss; d.a_k = 1;
+  d.tri = tri ? &flag : nullptr;
+  d.work = room ? reinterpret_cast<double2*>(16) : nullptr;
+  d.work_elems = room;
+  return gg::zgemm_choose(d, batch, (long)KB * ((K + 3) / 4), sms).splits;
+}
+
 // number of tile shapes; rows and columns of one and its teams per SM
 extern "C" int zgemm_shapes(int gauss) { return gauss ? gg::kZShapes3 : gg::kZShapes; }
 extern "C" void zgemm_tile(int gauss, int shape, int64_t* out) {
